@@ -876,12 +876,22 @@ int launch_band(Runner& R, int k) {
     CK(cudaMemsetAsync(B.band, 0, sizeof(double) * (size_t)B.n * B.width, R.stream));
     k_band_fill<<<nblk(c->nnzb, 256), 256, 0, R.stream>>>(B, c->blk_row.p, c->nnzb);
     k_band_rhs<<<nblk(c->V, 256), 256, 0, R.stream>>>(B);
-    k_band_factor<<<1, kBandThreads, 0, R.stream>>>(B);
-    k_band_solve<<<1, kBandThreads, 0, R.stream>>>(B);
+    // in panels while the band's window fits in shared memory (at every such width the faster one),
+    // else pivot by pivot in global memory
+    const bool window = B.bw <= kBandWindowMaxBw;
+    if (window) {
+        void* kern = band_window_kernel(B.bw);
+        void* args[] = {(void*)&B};
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)band_window_smem(kBandWindowMaxBw)));
+        CK(cudaLaunchKernel(kern, dim3(1), dim3(kBandWindowThreads), args, band_window_smem(B.bw), R.stream));
+    } else {
+        k_band_factor<<<1, kBandThreads, 0, R.stream>>>(B);
+        k_band_solve<<<1, kBandThreads, 0, R.stream>>>(B);
+    }
     k_band_apply<<<nblk(c->V, 256), 256, 0, R.stream>>>(B, c->H(0), c->U(0), c->Vv(0), c->sol.p,
                                                           R.ktab_h[k].K.apply_inc, R.ctl.p + k);
     CK(cudaGetLastError());
-    R.launches += 5;
+    R.launches += window ? 4 : 5;
     return 0;
 }
 
