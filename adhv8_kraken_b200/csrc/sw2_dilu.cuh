@@ -45,12 +45,71 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include "sw2_krylov.cuh"   // KrylovCtl, grid_sync, block_partial, grid_allreduce, inv3, LaunchMap
+#include "sw2_krylov.cuh"   // KrylovCtl, grid_sync, warp_combine, inv3, LaunchMap
 
 namespace sw2 {
 
-constexpr int kDiluThreads = 256;                   // = kKrylovRowThreads: the reduction helpers' CTA
+constexpr int kDiluThreads = 256;
 constexpr int kDiluWarps = kDiluThreads / 32;
+
+template <int N>
+struct IntC {
+    static constexpr int value = N;
+};
+
+// deterministic all-reduce of up to 4 per-block partials: every block combines the partials
+// of all blocks in the same fixed order (sum or max per slot); red = shared [4][kDiluWarps].
+// Called by the whole CTA.
+template <int NV>
+__device__ __forceinline__ void grid_allreduce(const double* part, int nparts, const int* is_max, double* out,
+                                               double* red) {
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    {
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            double a = 0.0;
+            for (int k = threadIdx.x; k < nparts; k += kDiluThreads) {
+                const double p = __ldcg(part + (size_t)k * 4 + q);
+                a = is_max[q] ? fmax(a, p) : a + p;
+            }
+            a = warp_combine(a, is_max[q]);
+            if (lane == 0) red[q * kDiluWarps + warp] = a;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        double a = red[q * kDiluWarps];
+#pragma unroll
+        for (int w = 1; w < kDiluWarps; w++) a = is_max[q] ? fmax(a, red[q * kDiluWarps + w]) : a + red[q * kDiluWarps + w];
+        out[q] = a;
+    }
+    __syncthreads();
+}
+
+// block partials: the threads' values combined in a fixed order, written by thread 0 to slot `slot`
+template <int NV>
+__device__ __forceinline__ void block_partial(double* vals, const int* is_max, double* part, int slot, double* red) {
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        const double a = warp_combine(vals[q], is_max[q]);
+        if (lane == 0) red[q * kDiluWarps + warp] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            double a = red[q * kDiluWarps];
+#pragma unroll
+            for (int w = 1; w < kDiluWarps; w++)
+                a = is_max[q] ? fmax(a, red[q * kDiluWarps + w]) : a + red[q * kDiluWarps + w];
+            part[(size_t)slot * 4 + q] = a;
+        }
+    }
+    __syncthreads();
+}
+
 constexpr int kMaxColours = 16;
 constexpr int kDiluVectors = 11;                    // x', r, r0, p, nu, t, t1, g, s, w, t2 (new order, [3V])
 constexpr int kDiluChunk = 4;                       // blocks of a row whose gathers are issued together
@@ -280,7 +339,7 @@ __device__ __forceinline__ void dl_row_sub(const MT* __restrict__ B, const int* 
 
 template <typename MT, class SRC>
 __global__ void __launch_bounds__(kDiluThreads, kDiluMinBlocks) k_dilu_bicgstab(const __grid_constant__ SRC srcs) {
-    __shared__ double red[4 * kKrylovWarps];
+    __shared__ double red[4 * kDiluWarps];
     int pl, np;
     double rtol;
     const DiluArgs& K = srcs.get(pl, np, rtol);

@@ -56,7 +56,8 @@ struct __align__(16) Inst {
     PhysParams P;
     double *sc, *sx, *sy;       // residual slots (3T + 2E each)
     double *R, *sol, *jslots, *val, *S, *bs, *dinv;
-    void* aoff;                 // folded off-diagonal blocks (MT of the Krylov launch)
+    void* aoff;                 // folded off-diagonal blocks (MT of the Krylov launch) in tile records
+    const int *boff, *orow;     // where tile m's blocks begin (16-byte units), off-diagonal row pointers
     unsigned char *ewet, *mark;
     int *glist, *gcount;
     int* ngen;                  // general-list length of the last residual evaluation (the
@@ -754,7 +755,7 @@ __global__ void k_rowscale(const __grid_constant__ Src src, int fix_only) {
 // and D_i the scaled diagonal block of row i, the Krylov operator M^-1 A' has identity
 // diagonal blocks and off-diagonal blocks D_i^-1 A'_ij, so the sweeps stream only those
 // (nnzb - V blocks, no inverses).  D_i^-1 comes from k_rowscale; the off-diagonal block k of
-// row i goes to position k - i - (k > dpos_i) of the folded matrix,
+// row i is off-diagonal block k - i - (k > dpos_i) and goes to its place in its tile's record,
 // D_i^-1 (S_i A_ij S_j) formed in FP64 and stored as MT
 template <class Src, typename MT>
 __global__ void k_fold_offdiag(const __grid_constant__ Src src) {
@@ -764,7 +765,6 @@ __global__ void k_fold_offdiag(const __grid_constant__ Src src) {
     const double* __restrict__ val = I.val;
     const double* __restrict__ S = I.S;
     const double* __restrict__ dinv = I.dinv;
-    MT* __restrict__ aoff = (MT*)I.aoff;
     const int k = lb * blockDim.x + threadIdx.x;
     if (k >= m.nnzb) return;
     const int i = m.blk_row[k], j = m.col[k];
@@ -777,7 +777,9 @@ __global__ void k_fold_offdiag(const __grid_constant__ Src src) {
         for (int c = 0; c < 3; c++) bq[3 * r + c] = val[(size_t)k * 9 + 3 * r + c] * (S[3 * i + r] * S[3 * j + c]);
 #pragma unroll
     for (int q = 0; q < 9; q++) d[q] = dinv[(size_t)i * 9 + q];
-    MT* o = aoff + (size_t)(k - i - (k > dp ? 1 : 0)) * 9;
+    const int tile = i / kTileRows;
+    MT* o = (MT*)((unsigned char*)I.aoff + 16 * (size_t)I.boff[tile]) +
+            (size_t)(k - i - (k > dp ? 1 : 0) - I.orow[tile * kTileRows]) * 9;
     fold_block(d, bq, o);
 }
 

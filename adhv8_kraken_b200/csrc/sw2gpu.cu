@@ -184,10 +184,10 @@ struct sw2gpu_ctx {
     // (orowptr / ocol: the BCSR pattern without its diagonal); FP64 or FP32 storage
     std::vector<int> orowptr_h;
     DBuf<int> orowptr, ocol;
-    DBuf<double> aoff64, dinv64;
-    DBuf<float> aoff32;
+    DBuf<unsigned char> aoff;       // tile records of the folded operator
+    DBuf<int> tile_off, blk_off;    // where each begins, and its blocks, in 16-byte units
+    DBuf<double> dinv64;
     DBuf<double> kv64[kKrylovVectors];
-    DBuf<double> part;
     DBuf<Norms> npart;
     DBuf<unsigned> ncounter;
     int krylov_grid = 0;            // virtual CTAs of the Krylov solve (its partial structure)
@@ -200,10 +200,14 @@ struct sw2gpu_ctx {
     int its_at[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int its_snap[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int its_prev[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    unsigned a_cap = 0, c_cap = 0;  // largest tile block / column-index ranges (staged sweeps)
+    unsigned a_cap = 0;             // largest tile record (staged sweeps)
+    // the shares of the staged sweeps (sw2_halo.h): sub-ranges per virtual CTA (0: staging does not
+    // fit), rows of the largest operand buffer, halo lists, block columns in the buffers
+    int halo_nsub = 0, halo_rows = 0;
+    DBuf<int> halo_ptr, halo_idx;
     // autotuned launch variants (sw2gpu_autotune): they change speed, never results
     int tune_jac_minb = 2;          // wet-Jacobian CTAs per SM the register budget is cut for
-    int tune_stages = 3;            // Krylov tile-ring depth (0: sweeps from global memory)
+    int tune_stages = -1;           // Krylov tile-ring depth (0: sweeps from global memory; -1: by occupancy)
     // polls of a Krylov grid-barrier / tile-copy wait before it gives up (0: the library's
     // defaults); sw2gpu_set_wait_limits
     long long wait_barrier = 0, wait_copy = 0;
@@ -269,23 +273,8 @@ namespace {
 
 enum PhaseKind { kPhJac = 0, kPhKrylov = 1, kPhResid = 2 };
 
-#ifndef SW2_MAX_STAGED_SMEM
-#define SW2_MAX_STAGED_SMEM (96 * 1024)   // dynamic shared memory allowed for the tile ring
-#endif
-constexpr size_t kMaxStagedSmem = SW2_MAX_STAGED_SMEM;
-
-// bytes per stage of the staged Krylov sweeps: the largest 16-byte-rounded block range and
-// column-index range of any tile of kTileRows rows, for matrix elements of esz bytes
-void stage_caps(const std::vector<int>& rp, int V, size_t esz, unsigned& a_cap, unsigned& c_cap) {
-    size_t am = 16, cm = 16;
-    for (int r0 = 0; r0 < V; r0 += kTileRows) {
-        const size_t k0 = (size_t)rp[r0], k1 = (size_t)rp[std::min(r0 + kTileRows, V)];
-        am = std::max(am, ((k1 * 9 * esz + 15) & ~size_t(15)) - ((k0 * 9 * esz) & ~size_t(15)));
-        cm = std::max(cm, ((k1 * 4 + 15) & ~size_t(15)) - ((k0 * 4) & ~size_t(15)));
-    }
-    a_cap = (unsigned)am;
-    c_cap = (unsigned)cm;
-}
+// dynamic shared memory of the staged sweeps: what an SM has for one CTA (227 KB) less the static part
+constexpr size_t kMaxStagedSmem = 218 * 1024;
 
 // largest band the direct solve accepts (bytes of the band of the scaled system)
 constexpr size_t kBandMaxBytes = size_t(2) << 30;
@@ -341,6 +330,7 @@ struct Runner {
     bool tab_pending = false;
     DBuf<Norms> norms;
     DBuf<KrylovCtl> ctl;
+    DBuf<double> part;            // published partials of every instance's Krylov solve
     DBuf<int> singular;
     Norms* norms_h = nullptr;     // pinned mirrors, one entry per instance
     KrylovCtl* ctl_h = nullptr;
@@ -348,7 +338,7 @@ struct Runner {
     int jac_minb = 2;             // wet-Jacobian variant in use (register budget for 1 or 2 CTAs per SM)
     int jac_ctas[2] = {0, 0};     // persistent wet-Jacobian grid per variant (co-resident CTAs)
     bool jac_ready = false;       // jac_ctas set (kernel attributes applied)
-    unsigned c_off = 0, r_off = 0, v_off = 0, stage_bytes = 0;
+    unsigned stage_bytes = 0, x_bytes = 0;
     size_t smem = 0;
     int capacity = 0;             // co-resident Krylov CTAs
     // Krylov rebalancing of host-driven batch launches: up to rb_rounds launches per solve; in
@@ -507,7 +497,8 @@ int runner_alloc(Runner& R, cudaStream_t stream, bool mixed, int cap) {
     R.stream = stream;
     R.mixed = mixed;
     R.cap = cap;
-    if (R.ktab.alloc(cap) || R.dtab.alloc(cap) || R.norms.alloc(cap) || R.ctl.alloc(cap) || R.singular.alloc(cap) ||
+    if (R.ktab.alloc(cap) || R.dtab.alloc(cap) || R.norms.alloc(cap) || R.ctl.alloc(cap) ||
+        R.part.alloc(cap * krylov_part_doubles(kMaxVirtual)) || R.singular.alloc(cap) ||
         R.kdone.alloc(Runner::kMaxRounds))
         return fail(SW2GPU_E_NOMEM, "batch tables");
     CK(cudaMemsetAsync(R.norms.p, 0, sizeof(Norms) * cap, stream));
@@ -536,35 +527,34 @@ int runner_set(Runner& R, const std::vector<sw2gpu_ctx*>& ctx) {
     for (auto* c : ctx)
         if ((c->p.precision == SW2GPU_MIXED) != R.mixed) return fail(SW2GPU_E_ARG, "a batch has one precision");
     R.ctx = ctx;
-    unsigned a_cap = 16, c_cap = 16;
+    unsigned a_cap = 16;
+    int x_rows = 0;
+    bool staged = true;
     const sw2gpu_ctx* big = nullptr;
     for (auto* c : ctx) {
         a_cap = std::max(a_cap, c->a_cap);
-        c_cap = std::max(c_cap, c->c_cap);
+        x_rows = std::max(x_rows, c->halo_rows);
+        staged &= c->halo_nsub > 0;
         if (!big || c->nnzb > big->nnzb) big = c;
     }
-    int want = big ? big->tune_stages : 3;
+    int want = !staged ? 0 : big ? big->tune_stages : -1;
     R.jac_minb = big ? big->tune_jac_minb : 2;
     auto fitting_variant = [&R] {   // a wet-Jacobian variant that does not fit yields to the other
         if (R.jac_ready && !R.jac_ctas[R.jac_minb - 1] && R.jac_ctas[2 - R.jac_minb]) R.jac_minb = 3 - R.jac_minb;
     };
     fitting_variant();
-    const unsigned c_off = a_cap, r_off = c_off + c_cap;
-    const unsigned v_off = r_off + ((unsigned)(kTileRows + 1) * 4u + 15u) / 16u * 16u;
-    const unsigned stage = (v_off + (unsigned)kMaxEpilogue * tile_vec_bytes<double>() + 127u) & ~127u;
-    if (want > 0 && (size_t)want * stage > kMaxStagedSmem) want = (size_t)2 * stage <= kMaxStagedSmem ? 2 : 0;
-    if (R.capacity > 0 && want == R.stages &&
-        (!want || (a_cap <= R.c_off && c_cap <= R.r_off - R.c_off)))
-        return 0;   // the current layout still holds every tile
+    // a layout that holds what the last one held stays at least as large (instances come and go)
+    const unsigned stage = std::max((a_cap + 127u) & ~127u, R.stage_bytes);
+    const unsigned x_bytes = std::max(stage_x_bytes(x_rows), R.x_bytes);
+    auto bytes = [&](int st) { return (size_t)(st - 1) * kKrylovGroups * stage + x_bytes; };
+    if (want < 0) want = 3;   // the deepest ring that fits: a CTA whose tiles all stay in it copies them once
+    if (want > 0 && bytes(want) > kMaxStagedSmem) want = bytes(2) <= kMaxStagedSmem ? 2 : 0;
+    if (R.capacity > 0 && want == R.stages && (!want || (a_cap <= R.stage_bytes && stage_x_bytes(x_rows) <= R.x_bytes)))
+        return 0;   // the current layout still holds every tile and operand
     R.stages = want;
-    R.c_off = R.r_off = R.v_off = R.stage_bytes = 0;
-    if (R.stages) {
-        R.c_off = c_off;
-        R.r_off = r_off;
-        R.v_off = v_off;
-        R.stage_bytes = stage;
-    }
-    R.smem = (size_t)R.stages * R.stage_bytes;
+    R.stage_bytes = R.stages ? stage : 0;
+    R.x_bytes = R.stages ? x_bytes : 0;
+    R.smem = R.stages ? bytes(R.stages) : 0;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -580,7 +570,7 @@ int runner_set(Runner& R, const std::vector<sw2gpu_ctx*>& ctx) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kone, kKrylovThreads, R.smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tab, ktab, kKrylovThreads, R.smem));
     per_sm = std::min(per_sm, per_sm_tab);
-    R.capacity = sms * std::max(1, std::min(per_sm, 4));
+    R.capacity = sms * std::max(1, std::min(per_sm, 1));
     if (!R.jac_ready) {
         R.jac_ready = true;
         // wet-Jacobian kernels: double-buffered records above the 48 KB static limit, and a
@@ -671,7 +661,9 @@ int runner_tables(Runner& R, int apply_inc) {
         I.sc = c->sc.p; I.sx = c->sx.p; I.sy = c->sy.p;
         I.R = c->R.p; I.sol = c->sol.p; I.jslots = c->jslots.p; I.val = c->val.p;
         I.S = c->S_.p; I.bs = c->bs.p; I.dinv = c->dinv64.p;
-        I.aoff = R.mixed ? (void*)c->aoff32.p : (void*)c->aoff64.p;
+        I.aoff = c->aoff.p;
+        I.boff = c->blk_off.p;
+        I.orow = c->orowptr.p;
         I.ewet = c->ewet.p; I.mark = c->mark.p; I.glist = c->glist.p; I.gcount = c->gcount.p; I.ngen = c->ngen.p;
         I.npart = c->npart.p; I.norms = R.norms.p + k; I.ncounter = c->ncounter.p; I.singular = R.singular.p + k;
         I.ndir = (int)c->dir_node.size();
@@ -683,6 +675,11 @@ int runner_tables(Runner& R, int apply_inc) {
         A.V = c->V;
         A.rowptr = c->orowptr.p;
         A.col = c->ocol.p;
+        A.nsub = c->halo_nsub;
+        A.hptr = c->halo_ptr.p;
+        A.hidx = c->halo_idx.p;
+        A.toff = c->tile_off.p;
+        A.boff = c->blk_off.p;
         A.S = c->S_.p;
         A.bs = c->bs.p;
         A.atol = c->p.lin_atol;
@@ -690,10 +687,9 @@ int runner_tables(Runner& R, int apply_inc) {
         A.h = c->H(0); A.u = c->U(0); A.v = c->Vv(0);
         A.sol = c->sol.p;
         A.apply_inc = apply_inc;
-        A.part = c->part.p;
+        A.part = R.part.p + (size_t)k * krylov_part_doubles(kMaxVirtual);
         A.ctl = R.ctl.p + k;
         A.vgrid = c->krylov_grid;
-        A.fuse_update = krylov_fuse_update(c->V);   // alone; a batch launch decides for its group
         A.spin_limit = c->wait_barrier;
         A.copy_limit = c->wait_copy;
         Q.A = I.aoff;
@@ -989,13 +985,14 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
         rc = launch_map(R, sub, 256, [&](int k) { return nblk(C(k)->nnzb, 256); }, SW2_GO_T(k_fold_offdiag, double));
     if (rc) return rc;
     CK(cudaMemsetAsync(R.ctl.p, 0, sizeof(KrylovCtl) * R.ctx.size(), R.stream));
+    CK(cudaMemsetAsync(R.part.p, 0, sizeof(double) * R.ctx.size() * krylov_part_doubles(kMaxVirtual), R.stream));
     Phase ph(&R, kPhKrylov);
     for (int k : band)
         if ((rc = launch_band(R, k))) return rc;
     if ((rc = launch_dilu(R, dl, eta))) return rc;
     // instances that cannot all be co-resident go in successive launches
     size_t j0 = 0;
-    const StageLayout lay{R.c_off, R.r_off, R.v_off, R.stage_bytes};
+    const StageLayout lay{R.stage_bytes, R.x_bytes};
     while (j0 < sub.size()) {
         std::vector<int> grp;
         for (size_t j = j0; j < sub.size() && (int)grp.size() < R.capacity; j++) grp.push_back(sub[j]);
@@ -1035,9 +1032,6 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
             }
             t.mp.boff[grp.size()] = off;
             t.lay = lay;
-            long long nodes = 0;
-            for (int k : grp) nodes += C(k)->V;
-            t.fuse = krylov_fuse_update(nodes);
             t.done_ctas = last ? nullptr : R.kdone.p + round;
             t.pause_after = (unsigned)std::ceil(R.rb_frac * total);
             t.resume = round > 0 ? 1 : 0;
@@ -2064,15 +2058,11 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
     rc |= zalloc(c->S_, 3ull * V, st); rc |= zalloc(c->bs, 3ull * V, st);
     rc |= zalloc(c->dinv64, 9ull * V, st);
     const bool bjacobi = prm->precond == SW2GPU_PREC_BJACOBI;   // the folded operator and its vectors
-    if (bjacobi && prm->precision == SW2GPU_MIXED)
-        rc |= zalloc(c->aoff32, 9ull * (nnzb - V), st);
-    else if (bjacobi)
-        rc |= zalloc(c->aoff64, 9ull * (nnzb - V), st);
+    std::vector<int> ocol;
     {
         // the pattern without its diagonal (one diagonal block per row, checked above)
         std::vector<int>& orp = c->orowptr_h;
         orp.assign(V + 1, 0);
-        std::vector<int> ocol;
         ocol.reserve(nnzb - V);
         for (int n = 0; n < V; n++) {
             for (int k = rp[n]; k < rp[n + 1]; k++)
@@ -2081,6 +2071,23 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
         }
         rc |= up(c->orowptr, orp, st);
         rc |= up(c->ocol, ocol, st);
+        if (bjacobi) {   // the tile records
+            const int nt = nblk(V, kTileRows), esz = prm->precision == SW2GPU_MIXED ? sizeof(float) : sizeof(double);
+            std::vector<int> toff(nt + 1, 0), boff(nt);
+            long long at = 0;
+            for (int m = 0; m < nt; m++) {
+                const int nb = orp[std::min(V, (m + 1) * kTileRows)] - orp[m * kTileRows];
+                const long long bytes = tile_bytes(nb, esz);
+                c->a_cap = (unsigned)std::max<long long>(c->a_cap, std::min<long long>(bytes, 1 << 30));
+                boff[m] = (int)(at + tile_head(nb) / 16);
+                at += bytes / 16;
+                toff[m + 1] = (int)at;
+            }
+            if (at > INT32_MAX) return fail(SW2GPU_E_NOMEM, "the folded operator exceeds 32 GiB");
+            rc |= up(c->tile_off, toff, st);
+            rc |= up(c->blk_off, boff, st);
+            rc |= zalloc(c->aoff, 16 * (size_t)at, st);
+        }
     }
     if (prm->precond == SW2GPU_PREC_BAND) {
         std::vector<int> perm;
@@ -2105,27 +2112,33 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
     const int gblocks = nblk(V, kGatherThreads);
     rc |= zalloc(c->npart, gblocks, st);
     if (rc) return rc;
-    // Krylov: the largest tile ranges (for the staged sweeps' stage layout) and the virtual
-    // grid, which is the co-resident grid this instance gets alone (it fixes the order of
-    // every Krylov reduction, so the instance's results do not depend on its batch)
-    {
-        const bool mixed = prm->precision == SW2GPU_MIXED;
-        const unsigned esz = mixed ? sizeof(float) : sizeof(double);
-        stage_caps(c->orowptr_h, V, esz, c->a_cap, c->c_cap);
-    }
     CK(cudaMallocHost(&c->stage_h, sizeof(double) * stage_doubles(c)));
     CK(cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming));
-    std::vector<sw2gpu_ctx*> me(1, c);
-    c->self.reset(new Runner());
-    if ((rc = runner_init(*c->self, me, st))) return rc;
-    // one virtual CTA per tile of kTileRows rows, at most kVirtualPerSM per SM: small meshes get
-    // many CTAs when batched (a Krylov launch lasts as long as its slowest instance).  Fixed by
-    // the device, not by the tuned occupancy: it sets the order of every Krylov reduction
+    // the virtual grid: fixed by the device, not by the launch variant, since it sets the order of
+    // every Krylov reduction (an instance's results do not depend on its batch)
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int ntiles = nblk(V, kTileRows);
-    c->krylov_grid = std::max(1, std::min(ntiles, kVirtualPerSM * sms));
-    if (zalloc(c->part, 8ull * c->krylov_grid, st)) return SW2GPU_E_NOMEM;
+    c->krylov_grid = krylov_vgrid(V, std::min(sms, kMaxVirtual));
+    if (bjacobi) {
+        HaloTables ht;
+        build_halo(V, c->orowptr_h.data(), ocol.data(), c->krylov_grid, kHaloCapRows, ht);
+        c->halo_nsub = ht.nsub;
+        c->halo_rows = ht.max_rows;
+        rc |= up(c->halo_ptr, ht.ptr, st);
+        rc |= up(c->halo_idx, ht.idx, st);
+        DBuf<unsigned short> lcol;   // only the records keep it
+        rc |= up(lcol, ht.lcol, st);
+        if (rc) return rc;
+        if (ht.nsub) {
+            k_tile_heads<<<nblk(32LL * nblk(V, kTileRows), 256), 256, 0, st>>>(V, c->orowptr.p, lcol.p, c->tile_off.p, c->aoff.p);
+            CK(cudaGetLastError());
+        }
+        CK(cudaStreamSynchronize(st));   // the tables go out of scope
+        c->bytes -= lcol.n * sizeof(unsigned short) + 16;
+    }
+    std::vector<sw2gpu_ctx*> me(1, c);
+    c->self.reset(new Runner());
+    if (rc || (rc = runner_init(*c->self, me, st))) return rc;
     DevMesh& d = c->dm;
     d.V = V; d.T = T; d.E = E; d.nnzb = nnzb;
     d.x = c->x.p; d.y = c->y.p; d.z = c->z.p;

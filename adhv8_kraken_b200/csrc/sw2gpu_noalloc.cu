@@ -38,21 +38,21 @@ namespace {
 constexpr double kSmall = 2.220446049250313e-16;   // DBL_EPSILON, the spv_jacobi floor
 constexpr int kMaxNodes = SW2GPU_NOALLOC_MAX_NODES;
 constexpr int kMaxBlocks = SW2GPU_NOALLOC_MAX_BLOCKS;
-constexpr int kMaxGrid = (kMaxNodes + kKrylovThreads - 1) / kKrylovThreads;   // persistent-kernel blocks
+constexpr int kNaVirtual = 160;   // virtual CTAs of a solve
 constexpr size_t kAlign = 32;                                                 // doubles = 256 bytes
 constexpr size_t al(size_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
 // layout (in doubles): control word, partials, S, b', Dinv, folded off-diagonal blocks, their
 // row pointers and column indices (int32, two per double), the Krylov vectors
 constexpr size_t kOffCtl = 0;
 constexpr size_t kOffPart = kOffCtl + al((sizeof(KrylovCtl) + 7) / 8);
-constexpr size_t kOffS = kOffPart + al(2ull * kMaxGrid * 4);
+constexpr size_t kOffS = kOffPart + al(krylov_part_doubles(kNaVirtual));
 constexpr size_t kOffB = kOffS + al(3ull * kMaxNodes);
 constexpr size_t kOffDinv = kOffB + al(3ull * kMaxNodes);
 constexpr size_t kOffA = kOffDinv + al(9ull * kMaxNodes);
 constexpr size_t kOffRp = kOffA + al(9ull * kMaxBlocks);
 constexpr size_t kOffCol = kOffRp + al((kMaxNodes + 2) / 2);
 constexpr size_t kOffVec = kOffCol + al((kMaxBlocks + 1) / 2);
-constexpr size_t kScratchDoubles = kOffVec + kKrylovVectors * al(3ull * kMaxNodes);
+constexpr size_t kScratchDoubles = kOffVec + (kKrylovVectors + 2) * al(3ull * kMaxNodes);
 static_assert(kScratchDoubles * sizeof(double) > 16650000 && kScratchDoubles * sizeof(double) < 16750000,
               "the work array is documented as 16.7 MB");
 // the structure-check word sits in the control region, after the KrylovCtl record
@@ -229,7 +229,7 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
     }
     // the control words (barrier counter, error and result fields, structure-check word) must
     // start at zero; everything else is written before it is read
-    if (cudaMemsetAsync(ctl, 0, kAlign * sizeof(double), st) != cudaSuccess)
+    if (cudaMemsetAsync(ctl, 0, (kOffS - kOffCtl) * sizeof(double), st) != cudaSuccess)   // and the partials
         return na_fail(SW2GPU_E_CUDA, "cudaMemsetAsync of the control words failed");
     const int nb = (nnodes + 255) / 256;
     k_na_check<<<nb, 256, 0, st>>>(nnodes, nnzb, row_ptr, col, check);
@@ -256,8 +256,7 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bicgstab<double, double, 0, KrylovOne>,
                                                            kKrylovThreads, 0)) != cudaSuccess)
         return na_fail(SW2GPU_E_CUDA, cudaGetErrorString(e));
-    const int grid = std::max(1, std::min({kMaxGrid, (nnodes + kKrylovThreads - 1) / kKrylovThreads,
-                                           sms * std::max(per_sm, 1)}));
+    const int grid = krylov_vgrid(nnodes, std::min(sms, kNaVirtual));
     // one instance, direct sweeps (no tile ring); the record is a kernel parameter
     static thread_local KrylovOne one;
     KrylovArgs& K = one.Q.K;
@@ -274,7 +273,9 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
     K.part = part;
     K.ctl = ctl;
     K.vgrid = grid;
-    K.fuse_update = krylov_fuse_update(nnodes);
+    K.nsub = 0;   // direct sweeps: no share tables
+    K.hptr = K.hidx = nullptr;
+    K.toff = K.boff = nullptr;   // blocks in pattern order
     K.spin_limit = 0;   // the library's default bounds on the device waits
     K.copy_limit = 0;
     one.Q.A = A;
@@ -282,7 +283,7 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
     for (int k = 0; k < kKrylovVectors; k++) one.Q.vec[k] = v[k];
     one.rtol = rtol;
     one.rtol_dev = nullptr;
-    one.lay = StageLayout{0, 0, 0, 0};
+    one.lay = StageLayout{0, 0};
     void* args[] = {(void*)&one};
     e = cudaLaunchCooperativeKernel((void*)k_bicgstab<double, double, 0, KrylovOne>, dim3(grid),
                                                 dim3(kKrylovThreads), args, 0, st);
