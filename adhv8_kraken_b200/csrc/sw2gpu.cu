@@ -178,6 +178,7 @@ struct sw2gpu_ctx {
     DBuf<int> glist, gcount;     // elements on the general (wet/dry) Jacobian path
     DBuf<int> ngen;              // its length at the last residual evaluation (device copy)
     int ngeneral = 0;            // its length at the last residual evaluation
+    bool wet_closed = false;     // the closed forms cover every material (sw2_wet_jac.cuh)
     // work
     DBuf<double> sc, sx, sy, R, sol, jslots, val, S_, bs;
     // Krylov operator: block-Jacobi inverse folded into the off-diagonal blocks
@@ -807,21 +808,28 @@ int read_results(Runner& R, const std::vector<int>& evaluated) {
     return rc ? rc : finish_results(R, evaluated);
 }
 
-int launch_jacobian(Runner& R, const std::vector<int>& sub) {
+// differences: the wet elements by the reference's differences too (sw2gpu_load); else by the closed
+// forms where an instance's materials allow
+int launch_jacobian(Runner& R, const std::vector<int>& sub, bool differences = false) {
     Phase ph(&R, kPhJac);
     auto C = [&](int k) { return R.ctx[k]; };
+    std::vector<int> closed, diff;
+    for (int k : sub) (C(k)->wet_closed && !differences ? closed : diff).push_back(k);
+    int rc = launch_map(R, closed, kJacClosedElems, [&](int k) { return nblk(C(k)->T, kJacClosedElems); },
+                        SW2_GO(k_jac_elem_closed<std::decay_t<decltype(src)>>));
+    if (rc) return rc;
     // the general list and the wet flags come from the residual evaluated at this same state
     auto wet_blocks = [&](int k) { return nblk(C(k)->T, kJacElems); };
     auto wet = [&](auto minb) {   // persistent: the grid walks the launch's nb_ element groups
         constexpr int MB = decltype(minb)::value;
-        return launch_map(R, sub, kJacWetThreads, wet_blocks, [&](const auto& src, int nb_, int th_) {
+        return launch_map(R, diff, kJacWetThreads, wet_blocks, [&](const auto& src, int nb_, int th_) {
             k_jac_elem_wet<std::decay_t<decltype(src)>, MB>
                 <<<std::min(nb_, R.jac_ctas[MB - 1]), th_, kJacWetSmem, R.stream>>>(src, nb_);
         });
     };
     if (!R.jac_ctas[R.jac_minb - 1])
         return fail(SW2GPU_E_CUDA, "wet-Jacobian variant %d does not fit on this device", R.jac_minb);
-    int rc = R.jac_minb == 1 ? wet(std::integral_constant<int, 1>{}) : wet(std::integral_constant<int, 2>{});
+    rc = R.jac_minb == 1 ? wet(std::integral_constant<int, 1>{}) : wet(std::integral_constant<int, 2>{});
     if (rc) return rc;
     // a captured launch covers the largest list (the kernel reads the list's length itself)
     if ((rc = launch_map(R, sub, kJacThreads,
@@ -1998,6 +2006,7 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
         mp.cor_speed = std::sin((kPi / 180.) * m->mat_coriolis[k]) * 2. * kEarthRotat;
         mp.has_source = (k < c->S && c->str_bc[k] == SW2GPU_BCT_WATER_SOURCE) ? 1 : 0;
     }
+    c->wet_closed = std::all_of(c->mats_h.begin(), c->mats_h.begin() + c->M, wet_jac_material);
     // BCSR pattern and reference-order gather lists (sw2_tables.h)
     c->tri_h.assign(tri, tri + 3ull * T);
     c->edg_h.assign(edg, edg + 2ull * E);
@@ -2919,7 +2928,7 @@ int sw2gpu_load(sw2gpu_ctx* c, int32_t* nnzb, int32_t* row_ptr, int32_t* col, do
     CK(cudaMemcpyAsync(c->ngen.p, c->gcount.p, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaMemsetAsync(c->gcount.p, 0, sizeof(int), c->stream));
     if ((rc = read_results(R, one))) return rc;
-    if ((rc = launch_jacobian(R, one))) return rc;
+    if ((rc = launch_jacobian(R, one, true))) return rc;
     if ((rc = launch_map(R, one, 256, [&](int) { return nblk(c->V, 256); }, SW2_GO(k_rowscale<std::decay_t<decltype(src)>>, 1)))) return rc;
     if (row_ptr) memcpy(row_ptr, c->rowptr_h.data(), sizeof(int) * (c->V + 1));
     if (col) memcpy(col, c->col_h.data(), sizeof(int) * c->nnzb);
