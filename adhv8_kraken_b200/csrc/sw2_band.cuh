@@ -9,8 +9,9 @@
 // (SW2GPU_PREC_BAND): the nodes are renumbered in reverse Cuthill-McKee order on the host, the
 // scaled system S A S is scattered into a row-major band of half-width bw (dofs), factored in
 // place without pivoting (as the reference's profile LU), and the two triangular solves give the
-// increment directly.  One CTA walks the n = 3V pivots in order; the threads share the rank-1
-// update of each pivot's bw x bw trailing block and each triangular solve's row updates.  The
+// increment directly.  A band whose factor window fits in shared memory (bw <= 136) is factored
+// in panels of eight pivots (k_band_window); a wider one is walked pivot by pivot from global
+// memory (k_band_factor, k_band_solve), the threads sharing each pivot's bw x bw update.  The
 // work is n bw^2 for the factor and n bw for a solve, so the path is for the small and medium
 // systems of the reference's test decks, not for the 1M-triangle meshes (where the band does not
 // fit in the limit sw2gpu_create applies).
