@@ -43,6 +43,7 @@ struct TrnElem {
 
 // the parts of the element residual that do not depend on the current concentration
 struct TrnPre {
+    ClipGeo clip;               // of the current depth, shared by every evaluation of the element
     double to[3], too[3];       // t(n) and t(n-1) temporal contributions
     double h_wd, vwx, vwy;      // wet-area averages of the depth and the velocity (full averages when wet)
     double factor;              // wet/dry factor of the current depth
@@ -68,7 +69,7 @@ __device__ __forceinline__ void trn_gradphi_dot_vbar(const double* gx, const dou
 
 // one level's temporal term (fe_2d_trns_temporal, :692-726, with the wrapped integrand
 // fe_2d_transport_wd_temporal_triangle, fe_2d_transport_wet_dry_integrations.c:86-99), times dtf
-__device__ __forceinline__ void trn_temporal(const double* x, const double* y, const double* h, const double* c,
+__device__ __forceinline__ void trn_temporal(const ClipGeo& cl, const double* x, const double* y, const double* h, const double* c,
                                              double djac, double dtf, double* out) {
     double r[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     auto integ = [&](const double* X, const double* Y, const double* H, const double*, const double*, double dj,
@@ -80,7 +81,7 @@ __device__ __forceinline__ void trn_temporal(const double* x, const double* y, c
 #pragma unroll
         for (int i = 0; i < 3; i++) q[i][0] += I[i];
     };
-    wd_apply<false>(x, y, h, nullptr, nullptr, djac, 1, r, integ);
+    wd_apply<false>(cl, x, y, h, nullptr, nullptr, djac, 1, r, integ);
 #pragma unroll
     for (int i = 0; i < 3; i++) out[i] = dtf * r[i][0];
 }
@@ -92,8 +93,14 @@ __device__ __forceinline__ void trn_prepare(const TrnElem& E, const TrnParams& P
         uc[i] = (E.u[i] + 0.0) * 1.0;   // (vel + vcf) * mfcf (:183-187)
         vc[i] = (E.v[i] + 0.0) * 1.0;
     }
-    trn_temporal(E.x, E.y, E.ho, E.co, E.djac, (-1.) * (1. + P.alpha), pre.to);
-    trn_temporal(E.x, E.y, E.hoo, E.coo, E.djac, (P.alpha / 2.), pre.too);
+    make_clip_geo(E.x, E.y, E.h, E.djac, pre.clip);
+    {
+        ClipGeo c;
+        make_clip_geo(E.x, E.y, E.ho, E.djac, c);
+        trn_temporal(c, E.x, E.y, E.ho, E.co, E.djac, (-1.) * (1. + P.alpha), pre.to);
+        make_clip_geo(E.x, E.y, E.hoo, E.djac, c);
+        trn_temporal(c, E.x, E.y, E.hoo, E.coo, E.djac, (P.alpha / 2.), pre.too);
+    }
     const double h_avg = avg3(E.h), u_avg = avg3(uc), v_avg = avg3(vc);
     double gux = 0, guy = 0, gvx = 0, gvy = 0;
 #pragma unroll
@@ -108,7 +115,7 @@ __device__ __forceinline__ void trn_prepare(const TrnElem& E, const TrnParams& P
     pre.vwx = u_avg;
     pre.vwy = v_avg;
     pre.factor = 1.0;
-    if (E.wd != 0) pre.factor = wd_average<false>(E.x, E.y, E.h, uc, vc, E.djac, pre.h_wd, pre.vwx, pre.vwy);
+    if (E.wd != 0) pre.factor = wd_average<false>(pre.clip, E.x, E.y, E.h, uc, vc, E.djac, pre.h_wd, pre.vwx, pre.vwy);
     // diffusion (:258-290): MP DF on the transverse entry, or the estimated eddy viscosity
     const double h_fric = fmax(h_avg, kSmall);
     const double rough = (E.ks > kSmall) ? drag_coef(h_fric, E.ks) : 0.0;
@@ -143,7 +150,7 @@ __device__ __forceinline__ void trn_elem_resid(const TrnElem& E, const TrnPre& p
         er[i] = 0.0;
     }
     double tn[3];
-    trn_temporal(E.x, E.y, E.h, c, E.djac, (1. + P.alpha / 2.), tn);
+    trn_temporal(pre.clip, E.x, E.y, E.h, c, E.djac, (1. + P.alpha / 2.), tn);
 #pragma unroll
     for (int i = 0; i < 3; i++) er[i] += tn[i];
 #pragma unroll
@@ -171,7 +178,7 @@ __device__ __forceinline__ void trn_elem_resid(const TrnElem& E, const TrnPre& p
 #pragma unroll
             for (int i = 0; i < 3; i++) q[i][0] += ix * GX[i] + iy * GY[i];
         };
-        wd_apply<false>(E.x, E.y, E.h, E.gx, E.gy, E.djac, 1, r, integ);
+        wd_apply<false>(pre.clip, E.x, E.y, E.h, E.gx, E.gy, E.djac, 1, r, integ);
 #pragma unroll
         for (int i = 0; i < 3; i++) er[i] += r[i][0];
     }
