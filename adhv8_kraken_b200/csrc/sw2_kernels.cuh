@@ -399,10 +399,11 @@ __device__ __forceinline__ void stage_elem(const DevMesh& m, const State& s, int
 // into the element's record g[81] in global memory, o holding only R(x + eps e_j)): R(x + eps e_j)
 // and R(x - eps e_j), the central difference, and the Dirichlet zeroing of the element matrix.
 // GENERAL = false: fully wet physics, with the parts the column leaves unperturbed read from
-// `pre`; GENERAL = true: full wet/dry physics.
+// `pre`; GENERAL = true: full wet/dry physics, the upper half-warp (half = 1) evaluating the - pass
+// of the elements of the lower one, which writes.
 template <bool GENERAL>
 __device__ __forceinline__ void jac_column(const DevMesh& m, const PhysParams& P, const StagedElem& S,
-                                           const WetPre* pre, int item, double* o, double* g = nullptr) {
+                                           const WetPre* pre, int item, double* o, double* g = nullptr, int half = 0) {
     const int b = item / 3, var = item % 3;  // var: 0 = u, 1 = v, 2 = h
     // only the current iterate (9 values) is private; everything else is read from the
     // staged element in shared memory
@@ -442,9 +443,10 @@ __device__ __forceinline__ void jac_column(const DevMesh& m, const PhysParams& P
     // far below the FD truncation error)
     const double ie2 = 1.0 / (2.0 * eps);
     // pass 0 stores R(x + eps e_j) in this thread's 9 output entries, pass 1 turns them
-    // into the central difference; one residual body is instantiated, not two
+    // into the central difference; one residual body is instantiated, not two.  GENERAL: this
+    // thread evaluates the pass of its half-warp only, and both halves meet in a shuffle.
 #pragma unroll 1
-    for (int pass = 0; pass < 2; pass++) {
+    for (int pass = GENERAL ? half : 0; pass < (GENERAL ? half + 1 : 2); pass++) {
         const double xv = pass == 0 ? cur + eps : cur - eps;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -457,17 +459,23 @@ __device__ __forceinline__ void jac_column(const DevMesh& m, const PhysParams& P
         double r[3][3];
         if (GENERAL) sw2_elem_resid(S.in, hc, uc, vc, S.wd, pv, P, M, S.df, r);
         else elem_resid_impl<true, true>(S.in, hc, uc, vc, S.wd, pv, P, M, S.df, r, pre, fix);
+        double rm[3][3];   // GENERAL, lower half: R(x - eps e_j) of the upper half
+        if (GENERAL) {
+#pragma unroll
+            for (int q = 0; q < 9; q++) rm[q / 3][q % 3] = __shfl_xor_sync(0xffffffffu, r[q / 3][q % 3], 16);
+            if (half) break;
+        }
 #pragma unroll
         for (int a = 0; a < 3; a++) {
 #pragma unroll
             for (int eq = 0; eq < 3; eq++) {
                 const int row = (eq == 0) ? 2 : eq - 1;  // block rows: x-mom, y-mom, continuity
                 double& slot = o[(3 * a + b) * 9 + 3 * row + var];
-                if (pass == 0) {
+                if (!GENERAL && pass == 0) {
                     slot = r[a][eq];
                     continue;
                 }
-                double val = (slot - r[a][eq]) * ie2;
+                double val = (GENERAL ? r[a][eq] - rm[a][eq] : slot - r[a][eq]) * ie2;
                 const bool aD = (Dm >> a) & 1u, bD = (Dm >> b) & 1u, aP = (Pm >> a) & 1u, bP = (Pm >> b) & 1u;
                 const bool zero = (aD && row < 2) || (bD && var < 2) || (aP && row == 2) || (bP && var == 2);
                 const bool one = (a == b) && ((aD && ((var == 0 && row == 0) || (var == 1 && row == 1))) ||
@@ -612,27 +620,35 @@ __global__ void __launch_bounds__(kJacClosedElems) k_jac_elem_closed(const __gri
 
 // Elements of the general list (some vertex dry at some level, or a wet/dry-flagged
 // element), full wet/dry physics; the list length is the one the last residual evaluation
-// recorded.  One CTA per 32 listed elements.
+// recorded.  One CTA per 16 listed elements: a warp is one column of them, the + pass in its
+// lower half and the - pass in its upper half.  The list of a wet/dry basin is short (hundreds of
+// elements) and an evaluation is a long serial chain, so the launch lasts as long as one thread
+// and most of the chip is idle: one evaluation per thread instead of two took the Jacobian phase
+// of a 7k-triangle wet/dry basin from 82 to 56 us.  A long list costs the same as before (the
+// evaluations per warp halve, the warps double).
+constexpr int kJacGeneralElems = 16;
 template <class Src>
 __global__ void __launch_bounds__(kJacThreads) k_jac_elem_general(const __grid_constant__ Src src) {
     int lb, nb;
     const Inst& I = src.get(lb, nb);
     const DevMesh m = I.m;
-    __shared__ StagedElem se[kJacElems];
-    __shared__ double out[kJacElems * 81];
-    __shared__ int eid[kJacElems];
-    const int count = *I.ngen;
-    const int e0 = lb * kJacElems;
-    const int lane = threadIdx.x % kJacElems;
-    const int item = threadIdx.x / kJacElems;
-    const int nel = min(kJacElems, count - e0);
-    if (item == 0) {
-        const int e = lane < nel ? I.glist[e0 + lane] : -1;
+    __shared__ StagedElem se[kJacGeneralElems];
+    __shared__ double out[kJacGeneralElems * 81];
+    __shared__ int eid[kJacGeneralElems];
+    const int e0 = lb * kJacGeneralElems;
+    const int nel = min(kJacGeneralElems, *I.ngen - e0);
+    if (nel <= 0) return;
+    // lanes past the end of the list repeat its last element, so every lane takes the shuffles
+    const int half = threadIdx.x % 32 / kJacGeneralElems;
+    const int lane = min((int)threadIdx.x % kJacGeneralElems, nel - 1);
+    const int item = threadIdx.x / 32;
+    if ((int)threadIdx.x < nel) {
+        const int e = I.glist[e0 + lane];
         eid[lane] = e;
-        if (e >= 0) stage_elem(m, I.s, e, se[lane]);
+        stage_elem(m, I.s, e, se[lane]);
     }
     __syncthreads();
-    if (eid[lane] >= 0) jac_column<true>(m, I.P, se[lane], nullptr, item, out + lane * 81);
+    jac_column<true>(m, I.P, se[lane], nullptr, item, out + lane * 81, nullptr, half);
     __syncthreads();
     for (int k = threadIdx.x; k < nel * 81; k += blockDim.x) I.jslots[(size_t)eid[k / 81] * 81 + k % 81] = out[k];
 }

@@ -833,7 +833,7 @@ int launch_jacobian(Runner& R, const std::vector<int>& sub, bool differences = f
     if (rc) return rc;
     // a captured launch covers the largest list (the kernel reads the list's length itself)
     if ((rc = launch_map(R, sub, kJacThreads,
-                         [&](int k) { return nblk(R.capturing ? C(k)->T : C(k)->ngeneral, kJacElems); },
+                         [&](int k) { return nblk(R.capturing ? C(k)->T : C(k)->ngeneral, kJacGeneralElems); },
                          SW2_GO(k_jac_elem_general<std::decay_t<decltype(src)>>))))
         return rc;
     if ((rc = launch_map(R, sub, 128, [&](int k) { return nblk(6LL * C(k)->E, 128); }, SW2_GO(k_jac_edge<std::decay_t<decltype(src)>>)))) return rc;
