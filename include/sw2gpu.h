@@ -123,7 +123,7 @@ typedef struct sw2gpu_stats {
     double  device_ms;                 /* device time of the call (CUDA events) */
     int32_t kernel_launches;           /* kernels launched by the call */
     int32_t wd_elems;                  /* elements with wd_flag != 0 after the step */
-    double  jac_ms;                    /* FD Jacobian element kernel (summed over Newton iterations) */
+    double  jac_ms;                    /* Jacobian element kernels (summed over Newton iterations) */
     double  krylov_ms;                 /* persistent BiCGSTAB kernel */
     double  resid_ms;                  /* residual element + gather kernels */
     double  other_ms;                  /* block gather, scaling, line search, init */
@@ -154,9 +154,11 @@ int sw2gpu_destroy(sw2gpu_ctx *ctx);
  * server is not remeshed. */
 int sw2gpu_remesh(sw2gpu_ctx *old, const sw2gpu_mesh *mesh, sw2gpu_ctx **out);
 /* Launch variants (no counterpart in the reference).  Two knobs change the speed of a step,
- * never its results: the register budget of the wet-Jacobian kernel (jac_minb: 1 or 2
- * resident CTAs per SM) and the depth of the Krylov kernel's shared-memory tile ring (stages:
- * 0 = sweeps read global memory, 2 or 3).  sw2gpu_autotune times every variant on the
+ * never its results: the register budget of the differenced wet-Jacobian kernel (jac_minb: 1
+ * or 2 resident CTAs per SM; Newton iterations differentiate fully wet elements of materials
+ * with isotropic user viscosity in closed form and do not launch it) and the depth of the
+ * Krylov kernel's shared-memory tile rings (stages: 0 = sweeps read global memory, 2 or 3 = one
+ * or two places per group of row warps).  sw2gpu_autotune times every variant on the
  * context's own mesh and current state (which it leaves as it found it) and keeps the
  * fastest; a batch uses the variants of its instance with the most blocks. */
 int sw2gpu_autotune(sw2gpu_ctx *ctx, int32_t *jac_minb, int32_t *stages);
@@ -176,8 +178,8 @@ int sw2gpu_set_graphs(sw2gpu_ctx *ctx, int32_t enable);
 /* device memory the context holds (bytes); no counterpart in the reference */
 int64_t sw2gpu_device_bytes(const sw2gpu_ctx *ctx);
 /* Bounds of the device waits (no counterpart in the reference, whose solver runs on one CPU
- * thread): the Krylov kernel's grid barriers and its tile-copy waits give up after this many
- * polls, set SW2GPU_E_TIMEOUT and return; the step then resets the current level to the old
+ * thread): the Krylov kernel's waits for a reduction's partials and its tile-copy waits give up
+ * after this many polls, set SW2GPU_E_TIMEOUT and return; the step then resets the current level to the old
  * one, like a failed step, and the context stays usable.  0 = the library's defaults (2^23 and
  * 2^20 polls, a few seconds and about a second).  Failure-detection tests set a few polls to
  * make a wait run out without any fault. */
@@ -325,7 +327,7 @@ int sw2gpu_step(sw2gpu_ctx *ctx, double dt, const double *series, sw2gpu_stats *
 /* Hot-path pieces, for parity checks against the reference units:
  *   sw2gpu_resid: fe_sw2_init-free residual at the current state (fe_sw2_resid);
  *                 writes resid[3*nnodes] and applies the dry-node velocity zeroing.
- *   sw2gpu_load:  FD Jacobian (fe_sw2_load incl. the tiny-diagonal fix) in BCSR form:
+ *   sw2gpu_load:  FD Jacobian of every element (fe_sw2_load incl. the tiny-diagonal fix) in BCSR form:
  *                 row_ptr[nnodes+1], col[nnzb], val[9*nnzb] (sorted columns), and the
  *                 residual after the fix in resid[3*nnodes].  Pass NULL to query nnzb. */
 int sw2gpu_set_dt(sw2gpu_ctx *ctx, double dt, const double *series);
