@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
             // a CTA's first virtual CTA has its tiles at hand (the quotients of 64 bits take longer
             // than a small share's products)
             const int ta = v == pl ? ta0 : tile0(v), nt = v == pl ? nt0 : tile0(v + 1) - ta;
-            const int nsub = STAGED ? K.nsub : 1;
+            const int nsub = max(K.nsub, 1);   // without staging too: the sub-ranges set the order of the sums
 #pragma unroll 1
             for (int sq = 0; sq < nsub; sq++) {
                 const int sb = back ? nsub - 1 - sq : sq;
