@@ -33,7 +33,8 @@ inline void build_halo(int V, const int* rp, const int* col, int vgrid, int cap_
     const int most = (nt + vgrid - 1) / vgrid;   // tiles of the largest virtual CTA
     std::vector<int> mark(V, -1), at(V);
     int stamp = 0;
-    for (int nsub = std::max(1, (most * kHaloTileRows + cap_rows - 1) / cap_rows); nsub <= most; nsub += std::max(1, nsub / 4)) {
+    // steps of a quarter, the last attempt the division into single tiles
+    for (int nsub = std::min(most, std::max(1, (most * kHaloTileRows + cap_rows - 1) / cap_rows));; nsub = std::min(most, nsub + std::max(1, nsub / 4))) {
         t.ptr.assign(1, 0);
         t.idx.clear();
         t.lcol.assign(rp[V], 0);
@@ -67,6 +68,7 @@ inline void build_halo(int V, const int* rp, const int* col, int vgrid, int cap_
             t.nsub = nsub;
             return;
         }
+        if (nsub >= most) break;
     }
     t = HaloTables();
 }
