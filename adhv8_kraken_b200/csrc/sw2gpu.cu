@@ -32,6 +32,7 @@
 #include "sw2_tables.h"
 #include "sw2_kernels.cuh"
 #include "sw2_krylov.cuh"
+#include "sw2_layout.h"
 #include "sw2_series.h"
 #include "sw2_shares.h"
 #include "trn_kernels.cuh"
@@ -335,12 +336,10 @@ struct Runner {
     DBuf<int> singular;
     Norms* norms_h = nullptr;     // pinned mirrors, one entry per instance
     KrylovCtl* ctl_h = nullptr;
-    int stages = 0;               // Krylov tile-ring depth in use (0: sweeps from global memory)
+    RingLayout ring;              // Krylov tile rings and operand buffer in use
     int jac_minb = 2;             // wet-Jacobian variant in use (register budget for 1 or 2 CTAs per SM)
     int jac_ctas[2] = {0, 0};     // persistent wet-Jacobian grid per variant (co-resident CTAs)
     bool jac_ready = false;       // jac_ctas set (kernel attributes applied)
-    unsigned stage_bytes = 0, x_bytes = 0;
-    size_t smem = 0;
     int capacity = 0;             // co-resident Krylov CTAs
     // Krylov rebalancing of host-driven batch launches: up to rb_rounds launches per solve; in
     // every launch but the last, once rb_frac of its CTAs have finished their instances, the
@@ -528,48 +527,35 @@ int runner_set(Runner& R, const std::vector<sw2gpu_ctx*>& ctx) {
     for (auto* c : ctx)
         if ((c->p.precision == SW2GPU_MIXED) != R.mixed) return fail(SW2GPU_E_ARG, "a batch has one precision");
     R.ctx = ctx;
-    unsigned a_cap = 16;
-    int x_rows = 0;
-    bool staged = true;
+    std::vector<RingNeed> needs;
     const sw2gpu_ctx* big = nullptr;
     for (auto* c : ctx) {
-        a_cap = std::max(a_cap, c->a_cap);
-        x_rows = std::max(x_rows, c->halo_rows);
-        staged &= c->halo_nsub > 0;
+        needs.push_back(RingNeed{!c->band && !c->dilu, c->a_cap, stage_x_bytes(c->halo_rows), c->halo_nsub > 0});
         if (!big || c->nnzb > big->nnzb) big = c;
     }
-    int want = !staged ? 0 : big ? big->tune_stages : -1;
     R.jac_minb = big ? big->tune_jac_minb : 2;
     auto fitting_variant = [&R] {   // a wet-Jacobian variant that does not fit yields to the other
         if (R.jac_ready && !R.jac_ctas[R.jac_minb - 1] && R.jac_ctas[2 - R.jac_minb]) R.jac_minb = 3 - R.jac_minb;
     };
     fitting_variant();
-    // a layout that holds what the last one held stays at least as large (instances come and go)
-    const unsigned stage = std::max((a_cap + 127u) & ~127u, R.stage_bytes);
-    const unsigned x_bytes = std::max(stage_x_bytes(x_rows), R.x_bytes);
-    auto bytes = [&](int st) { return (size_t)(st - 1) * kKrylovGroups * stage + x_bytes; };
-    if (want < 0) want = 3;   // the deepest ring that fits: a CTA whose tiles all stay in it copies them once
-    if (want > 0 && bytes(want) > kMaxStagedSmem) want = bytes(2) <= kMaxStagedSmem ? 2 : 0;
-    if (R.capacity > 0 && want == R.stages && (!want || (a_cap <= R.stage_bytes && stage_x_bytes(x_rows) <= R.x_bytes)))
+    const RingLayout ring = ring_layout(needs, big ? big->tune_stages : -1, kKrylovGroups, kMaxStagedSmem, R.ring);
+    if (R.capacity > 0 && ring.stages == R.ring.stages && ring.smem == R.ring.smem && ring.x_bytes == R.ring.x_bytes)
         return 0;   // the current layout still holds every tile and operand
-    R.stages = want;
-    R.stage_bytes = R.stages ? stage : 0;
-    R.x_bytes = R.stages ? x_bytes : 0;
-    R.smem = R.stages ? bytes(R.stages) : 0;
+    R.ring = ring;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // the dynamic shared-memory cap is an attribute of the kernel, shared by every runner:
     // set to the largest tile ring any runner may use
-    void* kone = R.mixed ? krylov_kernel<float, KrylovOne>(R.stages) : krylov_kernel<double, KrylovOne>(R.stages);
-    void* ktab = R.mixed ? krylov_kernel<float, KrylovTab>(R.stages) : krylov_kernel<double, KrylovTab>(R.stages);
-    if (R.stages) {
+    void* kone = R.mixed ? krylov_kernel<float, KrylovOne>(R.ring.stages) : krylov_kernel<double, KrylovOne>(R.ring.stages);
+    void* ktab = R.mixed ? krylov_kernel<float, KrylovTab>(R.ring.stages) : krylov_kernel<double, KrylovTab>(R.ring.stages);
+    if (R.ring.stages) {
         CK(cudaFuncSetAttribute(kone, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStagedSmem));
         CK(cudaFuncSetAttribute(ktab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStagedSmem));
     }
     int per_sm_tab = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kone, kKrylovThreads, R.smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tab, ktab, kKrylovThreads, R.smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kone, kKrylovThreads, R.ring.smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tab, ktab, kKrylovThreads, R.ring.smem));
     per_sm = std::min(per_sm, per_sm_tab);
     R.capacity = sms * std::max(1, std::min(per_sm, 1));
     if (!R.jac_ready) {
@@ -1000,7 +986,7 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
     if ((rc = launch_dilu(R, dl, eta))) return rc;
     // instances that cannot all be co-resident go in successive launches
     size_t j0 = 0;
-    const StageLayout lay{R.stage_bytes, R.x_bytes};
+    const StageLayout lay{R.ring.stage_bytes, R.ring.x_bytes};
     while (j0 < sub.size()) {
         std::vector<int> grp;
         for (size_t j = j0; j < sub.size() && (int)grp.size() < R.capacity; j++) grp.push_back(sub[j]);
@@ -1013,8 +999,8 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
             one.rtol_dev = R.capturing ? R.eta_dev.p + grp[0] : nullptr;
             one.lay = lay;
             void* args[] = {(void*)&one};
-            void* kern = R.mixed ? krylov_kernel<float, KrylovOne>(R.stages) : krylov_kernel<double, KrylovOne>(R.stages);
-            CK(cudaLaunchCooperativeKernel(kern, dim3(P[0]), dim3(kKrylovThreads), args, R.smem, R.stream));
+            void* kern = R.mixed ? krylov_kernel<float, KrylovOne>(R.ring.stages) : krylov_kernel<double, KrylovOne>(R.ring.stages);
+            CK(cudaLaunchCooperativeKernel(kern, dim3(P[0]), dim3(kKrylovThreads), args, R.ring.smem, R.stream));
             R.launches++;
             continue;
         }
@@ -1048,8 +1034,8 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
                 R.launches++;
             }
             void* args[] = {(void*)&t};
-            void* kern = R.mixed ? krylov_kernel<float, KrylovTab>(R.stages) : krylov_kernel<double, KrylovTab>(R.stages);
-            CK(cudaLaunchCooperativeKernel(kern, dim3(total), dim3(kKrylovThreads), args, R.smem, R.stream));
+            void* kern = R.mixed ? krylov_kernel<float, KrylovTab>(R.ring.stages) : krylov_kernel<double, KrylovTab>(R.ring.stages);
+            CK(cudaLaunchCooperativeKernel(kern, dim3(total), dim3(kKrylovThreads), args, R.ring.smem, R.stream));
             R.launches++;
             if (last) break;
             CK(cudaMemcpyAsync(R.ctl_h, R.ctl.p, sizeof(KrylovCtl) * R.ctx.size(), cudaMemcpyDeviceToHost, R.stream));
@@ -1394,7 +1380,7 @@ int ensure_batch_graphs(Runner& R, const std::vector<int>& all, Runner::BatchGra
         dts.push_back(c->dt);
     }
     for (auto& g : R.bgraphs)
-        if (g.lv == lv && g.dt == dts && g.jac_minb == R.jac_minb && g.stages == R.stages) {
+        if (g.lv == lv && g.dt == dts && g.jac_minb == R.jac_minb && g.stages == R.ring.stages) {
             *out = &g;
             return 0;
         }
@@ -1407,7 +1393,7 @@ int ensure_batch_graphs(Runner& R, const std::vector<int>& all, Runner::BatchGra
     g.lv = lv;
     g.dt = dts;
     g.jac_minb = R.jac_minb;
-    g.stages = R.stages;
+    g.stages = R.ring.stages;
     int rc = capture_graph(R, &g.start, &g.kernels_start, [&] {
         int r = launch_init(R, all);
         if (!r) r = launch_resid(R, all);
@@ -1433,7 +1419,7 @@ int ensure_batch_graphs(Runner& R, const std::vector<int>& all, Runner::BatchGra
 int ensure_graphs(sw2gpu_ctx* c) {
     Runner& R = *c->self;
     sw2gpu_ctx::StepGraph& G = c->graphs[c->lv[0]];
-    if (G.start && G.newton && G.dt == c->dt && G.jac_minb == R.jac_minb && G.stages == R.stages) return 0;
+    if (G.start && G.newton && G.dt == c->dt && G.jac_minb == R.jac_minb && G.stages == R.ring.stages) return 0;
     if (G.start) cudaGraphExecDestroy(G.start);
     if (G.newton) cudaGraphExecDestroy(G.newton);
     G = sw2gpu_ctx::StepGraph();
@@ -1454,7 +1440,7 @@ int ensure_graphs(sw2gpu_ctx* c) {
     }
     G.dt = c->dt;
     G.jac_minb = R.jac_minb;
-    G.stages = R.stages;
+    G.stages = R.ring.stages;
     return 0;
 }
 
@@ -1592,7 +1578,7 @@ NewtonParams newton_params(const sw2gpu_ctx* c) {
 int ensure_loop_graph(sw2gpu_ctx* c) {
     Runner& R = *c->self;
     sw2gpu_ctx::StepGraph& G = c->graphs[c->lv[0]];
-    if (G.loop && G.dt == c->dt && G.jac_minb == R.jac_minb && G.stages == R.stages && G.loop_mass == c->mass_on)
+    if (G.loop && G.dt == c->dt && G.jac_minb == R.jac_minb && G.stages == R.ring.stages && G.loop_mass == c->mass_on)
         return 0;
     if (G.loop) cudaGraphExecDestroy(G.loop);
     G.loop = nullptr;
@@ -1702,7 +1688,7 @@ int ensure_loop_graph(sw2gpu_ctx* c) {
     }
     G.dt = c->dt;
     G.jac_minb = R.jac_minb;
-    G.stages = R.stages;
+    G.stages = R.ring.stages;
     G.loop_mass = c->mass_on;
     return 0;
 }
@@ -2967,7 +2953,7 @@ int sw2gpu_set_variant(sw2gpu_ctx* c, int32_t jac_minb, int32_t stages) {
 int sw2gpu_get_variant(const sw2gpu_ctx* c, int32_t* jac_minb, int32_t* stages) {
     if (!c) return fail(SW2GPU_E_ARG, "null context");
     if (jac_minb) *jac_minb = c->self->jac_minb;
-    if (stages) *stages = c->self->stages;
+    if (stages) *stages = c->self->ring.stages;
     return SW2GPU_OK;
 }
 
@@ -3024,7 +3010,7 @@ int sw2gpu_autotune(sw2gpu_ctx* c, int32_t* jac_minb, int32_t* stages) {
         if (rc) break;
         c->tune_stages = sg;
         if ((rc = runner_set(R, R.ctx))) break;
-        if (R.stages != sg) continue;   // this mesh's tiles do not fit that ring
+        if (R.ring.stages != sg) continue;   // this mesh's tiles do not fit that ring
         float t = 1e30f;
         if ((rc = timed([&] { return launch_linear(R, one, eta); }, t))) break;
         if (t < tb) { tb = t; best_s = sg; }
@@ -3039,7 +3025,7 @@ int sw2gpu_autotune(sw2gpu_ctx* c, int32_t* jac_minb, int32_t* stages) {
     CK(cudaStreamSynchronize(st));
     if (rc) return rc;
     if (jac_minb) *jac_minb = R.jac_minb;
-    if (stages) *stages = R.stages;
+    if (stages) *stages = R.ring.stages;
     return SW2GPU_OK;
 }
 
