@@ -32,20 +32,26 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <type_traits>
 
 #include "sw2_halo.h"
 
 namespace sw2 {
 
-// One CTA per SM: 15 row warps (SpMV rows, vector updates, partials) and one copy warp that fills
+// A CTA: 15 row warps (SpMV rows, vector updates, partials) and one copy warp that fills
 // the tile ring.  Three warps take a 32-row tile, one thread per component of a row: a thread's
 // products need no shuffles and its row's operands, result and dot products are coalesced.  (Eight
 // lanes per row in three CTAs of eight warps spent 2,600 cycles on a tile, most of it the latency
-// of shuffles and of three-component epilogues on one lane in eight.)  One CTA per SM also means a
-// third of the arrivals at every grid barrier.  Five groups of three warps: with 128 registers a
-// thread nothing spills, and spilled registers are lost from L1 at every barrier (six groups 1 to 3 %
-// slower, eight 10 %, four equal on small meshes and 2 % slower on 1M triangles).
+// of shuffles and of three-component epilogues on one lane in eight.)  Five groups of three warps:
+// with 128 registers a thread nothing spills, and spilled registers are lost from L1 at every barrier
+// (six groups 1 to 3 % slower, eight 10 %, four equal on small meshes and 5 % slower on 100k nodes).
+// Two forms of the same code: one CTA per SM, the shortest chain between two barriers, while that
+// gives every virtual CTA an SM; two per SM (64 registers, shallower rings) for batches and large
+// meshes, where an SM would otherwise stand still while its one CTA fills an operand buffer or waits
+// (Krylov time of a 256-member ensemble of 5k to 200k triangles, FP64 / mixed: 1,177 / 854 ms with one
+// CTA per SM, 859 / 558 with two; 64 members 314 / 221 and 227 / 148; 256 members of 2k to 10k 110
+// and 67).  Both compute the same bits.
 constexpr int kTileRows = 32;
 constexpr int kTileThreads = 3 * kTileRows;
 constexpr int kKrylovGroups = 5;                                 // tiles in work at once
@@ -70,12 +76,20 @@ constexpr bool kAlternate = true;
 // two tiles each up to 128 tiles, whose solves are launched alone more often and where a tile's own
 // time counts (the 4k channel: 11.4 us per iteration with two, 12.0 with five; 7k triangles 13.3 and
 // 15.1; from 500 tiles on within 3 %).
-inline int krylov_vgrid(int V, int sms) {
+// At most one per SM, two from pair_rows rows on (kPairRows): there an iteration is no longer the
+// latency of its barriers but the traffic of its sweeps, and two CTAs on an SM fill their operands
+// and multiply at different times.
+inline int krylov_vgrid(int V, int sms, int pair_rows = INT_MAX) {
     const int nt = (V + kTileRows - 1) / kTileRows;
     const int per = nt <= 128 ? 2 : kKrylovGroups;
-    const int v = (nt + per - 1) / per;
-    return v < 1 ? 1 : v > sms ? sms : v;
+    const int v = (nt + per - 1) / per, most = V >= pair_rows ? 2 * sms : sms;
+    return v < 1 ? 1 : v > most ? most : v;
 }
+// Where a mesh on its own gets two virtual CTAs per SM, by measurement (us per iteration, one and
+// two): FP64 100k nodes 33.3 and 34.1, 250k 72.6 and 74.1, 500k 145 and 140; mixed 100k 33.0 and 33.7,
+// 130k 40.5 and 38.4, 250k 73.2 and 64.0, 2M 570 and 433.
+template <typename MT>
+constexpr int kPairRows = sizeof(MT) == 4 ? 120000 : 300000;
 
 // Blocks of one launch over a batch: instance ids[j] owns blocks boff[j] .. boff[j+1]-1.
 // Passed by value (kernel parameter space), so lookups are uniform constant-bank reads.
@@ -308,10 +322,9 @@ struct StageLayout {
     unsigned stage_bytes, x_bytes;
 };
 __host__ __device__ constexpr unsigned stage_x_bytes(int rows) { return ((unsigned)rows * 24u + 127u) & ~127u; }
-// the largest operand buffer (48 KB): the 3,400 rows a virtual CTA of the 1M-triangle basin has and
-// their halo in two sub-ranges, beside a ring of ten tiles (three sub-ranges: 141.2 us per iteration
-// against 138.0)
-constexpr int kHaloCapRows = 2048;
+// the largest operand buffer (24 KB): with two CTAs on an SM what is left beside a ring of five tiles
+// each; the 1,700 rows a virtual CTA of the 1M-triangle basin has and their halo in two sub-ranges
+constexpr int kHaloCapRows = 1024;
 constexpr int kHaloKeep = 1024;   // halo rows whose numbers a CTA with one sub-range keeps in shared memory
 
 // Where a Krylov launch finds its instances.  KrylovOne: one instance, its record and
@@ -494,14 +507,21 @@ __device__ __forceinline__ VT row_apply(int c, int kb, int ke, BLK blk, CIX cix,
 // STAGES > 0: the row warps read the operand from the buffer in shared memory and the matrix from
 // a ring of STAGES - 1 tiles per warp group filled by bulk copies of the copy warp (completion on an
 // mbarrier per tile, release on another); the operands of large matrices' rows stay in L2
-// (policy_stream).  STAGES = 0: the threads load blocks and operands from global memory (meshes
+// (policy_stream).  PER_SM: CTAs that share an SM.  STAGES = 0: the threads load blocks and operands from global memory (meshes
 // whose tiles or halos do not fit).  Every variant computes the same bits.
 //
 // Measured (B200, us per iteration, with eight lanes per row, operands gathered from L2, three copies
-// per tile and a counter barrier before): 4k-triangle channel 12.7 -> 11.4, 32k mixed 23 -> 15.7, 200k
-// 48 -> 31.2, 260k mixed 55 -> 37.4, 1M 134 -> 138.  An iteration of the 1M basin moves 444 MB of matrix
-// and 156 MB of vectors (92 us at the measured copy rate); one of the 200k basin spends half its time in
-// the latency of its two sweeps' chains: operands, products, sums, fence, poll.
+// per tile and a counter barrier before): 4k-triangle channel 12.6 -> 11.1, 32k mixed 24 -> 16.8, 200k
+// 52 -> 33.3, 260k mixed 59 -> 38.4, 1M 140 -> 140, 4M mixed 492 -> 433.  An iteration of the 1M basin
+// moves 444 MB of matrix and 156 MB of vectors (92 us at the measured copy rate); one of the 200k basin
+// spends half its time in the latency of its two sweeps' chains: operands, products, sums, fence, poll.
+// Entries are numbered in 32 bits: 64-bit indices cost the two-CTA form spills (batches 3 % slower) and
+// both the extra instructions (200k 34.9 -> 33.3).
+// STAGES of direct sweeps over a pattern without share tables
+constexpr int kStagesWhole = -1;
+// places of a warp group's ring with two CTAs per SM
+template <typename MT>
+__host__ __device__ constexpr int pair_places() { return sizeof(MT) == 4 ? 2 : 1; }
 // what the row warps do next, and the scalars it takes
 enum KrylovNext : int { kSweepInit, kSweepPlain, kSweepUpdate, kSweepS, kSweepEnd, kSweepPause, kSweepFail };
 struct KrylovState {
@@ -510,8 +530,8 @@ struct KrylovState {
     unsigned nred;   // reductions so far: their number, and the buffer in turn
 };
 
-template <typename MT, typename VT, int STAGES, class KS>
-__global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_constant__ KS src) {
+template <typename MT, typename VT, int STAGES, int PER_SM, class KS>
+__global__ void __launch_bounds__(kKrylovThreads, PER_SM) k_bicgstab(const __grid_constant__ KS src) {
     __shared__ double red[3 * kKrylovWarps];    // a virtual CTA's sums, per warp
     __shared__ KrylovState C;                   // the solve's scalars and the next sweep
     __shared__ int s_hidx[STAGES > 0 ? kHaloKeep : 1];   // the halo rows of a CTA with one sub-range
@@ -665,8 +685,8 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
     unsigned tc = 0;     // tiles this group has taken: its place tc % S, mbarrier parity (tc / S) & 1
     bool wait_failed = false;
     using V2 = typename std::conditional<sizeof(VT) == 8, double2, float2>::type;
-    auto ld2 = [](const VT* p, size_t k) { return __ldcg(reinterpret_cast<const V2*>(p + k)); };
-    auto st2 = [](VT* p, size_t k, V2 v) { *reinterpret_cast<V2*>(p + k) = v; };
+    auto ld2 = [](const VT* p, unsigned k) { return __ldcg(reinterpret_cast<const V2*>(p + k)); };
+    auto st2 = [](VT* p, unsigned k, V2 v) { *reinterpret_cast<V2*>(p + k) = v; };
     if (tid == 0) {
         C.next = kSweepInit;
         if (src.resuming()) {   // the scalars of the paused solve (written by the previous launch)
@@ -718,15 +738,15 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
         };
         auto newu = [&](VT u, VT ap, VT p, VT r) { return fmadd(om, fmadd(-al, ap, r), fmadd(al, p, u)); };
         // the sweep's operand at entry e
-        auto operand = [&](size_t e) -> VT {
+        auto operand = [&](unsigned e) -> VT {
             if (mode == kSweepUpdate) {
                 VT rk;
                 return newp(ldv(apo + e), ldv(po + e), ldv(ro + e), ldv(As + e), rk);
             }
             if (mode == kSweepS) return fmadd(-al, ldv(apo + e), ldv(ro + e));
             if (mode == kSweepPlain) return ldv(po + e);
-            const size_t i = e / 3;   // b = M^-1 b': row e - 3 i of node i's inverse
-            const double* d = KI.Dinv + 3 * e;
+            const unsigned i = e / 3;   // b = M^-1 b': row e - 3 i of node i's inverse
+            const double* d = KI.Dinv + 3 * (size_t)e;
             const double* b = K.bs + 3 * i;
             return (VT)(d[0] * b[0] + d[1] * b[1] + d[2] * b[2]);
         };
@@ -740,17 +760,18 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
             // a CTA's first virtual CTA has its tiles at hand (the quotients of 64 bits take longer
             // than a small share's products)
             const int ta = v == pl ? ta0 : tile0(v), nt = v == pl ? nt0 : tile0(v + 1) - ta;
-            const int nsub = max(K.nsub, 1);   // without staging too: the sub-ranges set the order of the sums
+            // without staging too: the sub-ranges set the order of the sums
+            const int nsub = STAGES == kStagesWhole ? 1 : max(K.nsub, 1);
 #pragma unroll 1
             for (int sq = 0; sq < nsub; sq++) {
                 const int sb = back ? nsub - 1 - sq : sq;
                 const int ma = nsub == 1 ? ta : ta + sb * nt / nsub, mb = nsub == 1 ? ta + nt : ta + (sb + 1) * nt / nsub;
                 if (mb == ma) continue;
                 const int r0 = ma * kTileRows, n3 = 3 * (min(V, mb * kTileRows) - r0);
-                const size_t base = (size_t)r0 * 3;   // a multiple of 96: pairs are 16-byte aligned
+                const unsigned base = 3u * (unsigned)r0;   // a multiple of 96: pairs are 16-byte aligned
                 // q one tile ahead: its trip to L2 passes under the operand's, then under a tile's products
                 auto load_q = [&](int m) {
-                    return mode != kSweepInit && m >= ma && m < mb && m * kTileRows + li < V ? ldv(q + (size_t)m * kTileThreads + gt) : (VT)0;
+                    return mode != kSweepInit && m >= ma && m < mb && m * kTileRows + li < V ? ldv(q + (unsigned)(m * kTileThreads + gt)) : (VT)0;
                 };
                 const int first = back ? mb - 1 - group : ma + group, step = back ? -kKrylovGroups : kKrylovGroups;
                 VT qnext = load_q(first);
@@ -765,7 +786,7 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
                     VT* const un = KI.vec[C.ucur ^ C.pending];
 #pragma unroll 1
                     for (int k = tid; k < n2; k += kKrylovRowThreads) {
-                        const size_t e = base + 2 * (size_t)k;
+                        const unsigned e = base + 2u * (unsigned)k;
                         const V2 a = ld2(apo, e), p = ld2(po, e), r = ld2(ro, e), s = ld2(As, e), u = ld2(uo, e);
                         V2 uk, rk, pk;
                         uk.x = newu(u.x, a.x, p.x, r.x);
@@ -796,7 +817,7 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
 #pragma unroll 1
                     for (int t = kKrylovRowThreads - 1 - tid; t < nh; t += kKrylovRowThreads) {
                         const int h = t / 3, j = single ? s_hidx[h] : __ldg(K.hidx + h0 + h);
-                        xs[n3 + t] = operand((size_t)j * 3 + (t - 3 * h));
+                        xs[n3 + t] = operand((unsigned)(j * 3 + (t - 3 * h)));
                     }
                 }
                 bar_rows();
@@ -804,7 +825,7 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
                 for (int m = first; m >= ma && m < mb; m += step) {
                     const int i = m * kTileRows + li;
                     const bool act = i < V;
-                    const size_t e = (size_t)m * kTileThreads + gt;   // = 3 i + comp
+                    const unsigned e = (unsigned)(m * kTileThreads + gt);   // = 3 i + comp
                     const VT qe = qnext;
                     qnext = load_q(m + step);
                     VT y = 0, x = 0;
@@ -855,7 +876,7 @@ __global__ void __launch_bounds__(kKrylovThreads, 1) k_bicgstab(const __grid_con
                             [&](int k) { return __ldg(K.col + k); },
                             [&](int j, VT(&xj)[3]) {
 #pragma unroll
-                                for (int c = 0; c < 3; c++) xj[c] = operand((size_t)3 * j + c);
+                                for (int c = 0; c < 3; c++) xj[c] = operand((unsigned)(3 * j + c));
                             });
                         x = operand(e);
                     }

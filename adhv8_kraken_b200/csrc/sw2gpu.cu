@@ -277,17 +277,21 @@ enum PhaseKind { kPhJac = 0, kPhKrylov = 1, kPhResid = 2 };
 
 // dynamic shared memory of the staged sweeps: what an SM has for one CTA (227 KB) less the static part
 constexpr size_t kMaxStagedSmem = 218 * 1024;
+constexpr size_t kMaxPairSmem = 106 * 1024;   // the same of half an SM
 
 // largest band the direct solve accepts (bytes of the band of the scaled system)
 constexpr size_t kBandMaxBytes = size_t(2) << 30;
 
+// the Krylov kernel with two CTAs per SM
+template <typename MT, class KS>
+void* krylov_pair_kernel() { return (void*)k_bicgstab<MT, double, 1 + pair_places<MT>(), 2, KS>; }
 // Krylov kernel with a tile ring of `stages` stages (0: sweeps read global memory)
 template <typename MT, class KS>
 void* krylov_kernel(int stages) {
     switch (stages) {
-        case 2: return (void*)k_bicgstab<MT, double, 2, KS>;
-        case 3: return (void*)k_bicgstab<MT, double, 3, KS>;
-        default: return (void*)k_bicgstab<MT, double, 0, KS>;
+        case 2: return (void*)k_bicgstab<MT, double, 2, 1, KS>;
+        case 3: return (void*)k_bicgstab<MT, double, 3, 1, KS>;
+        default: return (void*)k_bicgstab<MT, double, 0, 1, KS>;
     }
 }
 
@@ -340,7 +344,9 @@ struct Runner {
     int jac_minb = 2;             // wet-Jacobian variant in use (register budget for 1 or 2 CTAs per SM)
     int jac_ctas[2] = {0, 0};     // persistent wet-Jacobian grid per variant (co-resident CTAs)
     bool jac_ready = false;       // jac_ctas set (kernel attributes applied)
-    int capacity = 0;             // co-resident Krylov CTAs
+    int capacity = 0;             // co-resident Krylov CTAs, one per SM
+    size_t pair_smem = 0;         // the same with two per SM
+    int pair_capacity = 0;        // 0: two do not fit
     // Krylov rebalancing of host-driven batch launches: up to rb_rounds launches per solve; in
     // every launch but the last, once rb_frac of its CTAs have finished their instances, the
     // instances still running pause and the next launch shares all CTAs among them
@@ -542,22 +548,34 @@ int runner_set(Runner& R, const std::vector<sw2gpu_ctx*>& ctx) {
     if (R.capacity > 0 && ring.stages == R.ring.stages && ring.smem == R.ring.smem && ring.x_bytes == R.ring.x_bytes)
         return 0;   // the current layout still holds every tile and operand
     R.ring = ring;
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // the dynamic shared-memory cap is an attribute of the kernel, shared by every runner:
-    // set to the largest tile ring any runner may use
-    void* kone = R.mixed ? krylov_kernel<float, KrylovOne>(R.ring.stages) : krylov_kernel<double, KrylovOne>(R.ring.stages);
-    void* ktab = R.mixed ? krylov_kernel<float, KrylovTab>(R.ring.stages) : krylov_kernel<double, KrylovTab>(R.ring.stages);
-    if (R.ring.stages) {
-        CK(cudaFuncSetAttribute(kone, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStagedSmem));
-        CK(cudaFuncSetAttribute(ktab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStagedSmem));
+    // co-resident CTAs per SM of a kernel and its batch form.  The dynamic shared-memory cap is an
+    // attribute of the kernel, shared by every runner: set to the most any runner may use
+    auto resident = [](void* one, void* tab, size_t smem, size_t cap, int& n) -> int {
+        int a = 0, b = 0;
+        CK(cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        CK(cudaFuncSetAttribute(tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, one, kKrylovThreads, smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, tab, kKrylovThreads, smem));
+        n = std::min(a, b);
+        return 0;
+    };
+    int per_sm = 0, rc = 0;
+    void* kone = R.mixed ? krylov_kernel<float, KrylovOne>(ring.stages) : krylov_kernel<double, KrylovOne>(ring.stages);
+    void* ktab = R.mixed ? krylov_kernel<float, KrylovTab>(ring.stages) : krylov_kernel<double, KrylovTab>(ring.stages);
+    if ((rc = resident(kone, ktab, ring.smem, ring.stages ? kMaxStagedSmem : 0, per_sm))) return rc;
+    if (per_sm < 1) return fail(SW2GPU_E_CUDA, "the Krylov solve kernel does not fit on this device");
+    R.capacity = sms;
+    R.pair_smem = (size_t)(R.mixed ? pair_places<float>() : pair_places<double>()) * kKrylovGroups * ring.stage_bytes + ring.x_bytes;
+    R.pair_capacity = 0;
+    if (ring.stages && R.pair_smem <= kMaxPairSmem) {
+        kone = R.mixed ? krylov_pair_kernel<float, KrylovOne>() : krylov_pair_kernel<double, KrylovOne>();
+        ktab = R.mixed ? krylov_pair_kernel<float, KrylovTab>() : krylov_pair_kernel<double, KrylovTab>();
+        if ((rc = resident(kone, ktab, R.pair_smem, kMaxPairSmem, per_sm))) return rc;
+        if (per_sm >= 2) R.pair_capacity = 2 * sms;
     }
-    int per_sm_tab = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kone, kKrylovThreads, R.ring.smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tab, ktab, kKrylovThreads, R.ring.smem));
-    per_sm = std::min(per_sm, per_sm_tab);
-    R.capacity = sms * std::max(1, std::min(per_sm, 1));
     if (!R.jac_ready) {
         R.jac_ready = true;
         // wet-Jacobian kernels: double-buffered records above the 48 KB static limit, and a
@@ -830,7 +848,7 @@ int launch_jacobian(Runner& R, const std::vector<int>& sub, bool differences = f
 // Krylov CTAs per instance: shares of the co-resident capacity by expected work (blocks x
 // iterations of the instance's last solve), at least one, at most its virtual CTAs, so that
 // the instances of a launch finish together
-std::vector<int> krylov_shares(Runner& R, const std::vector<int>& sub, const std::vector<int>* done = nullptr) {
+std::vector<int> krylov_shares(Runner& R, const std::vector<int>& sub, int capacity, const std::vector<int>* done = nullptr) {
     // the min-max allocation of sw2_shares.h over the instances' predicted work (done[k]:
     // iterations a resumed solve has behind it)
     const int n = (int)sub.size();
@@ -841,7 +859,7 @@ std::vector<int> krylov_shares(Runner& R, const std::vector<int>& sub, const std
         W[j] = krylov_work(c->nnzb, c->pred_its, done ? (*done)[sub[j]] : 0);
         G[j] = c->krylov_grid;
     }
-    return krylov_shares_minmax(W, G, R.capacity);
+    return krylov_shares_minmax(W, G, capacity);
 }
 
 // scaling, preconditioner folding and the persistent BiCGSTAB of the subset, each instance
@@ -987,21 +1005,36 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
     // instances that cannot all be co-resident go in successive launches
     size_t j0 = 0;
     const StageLayout lay{R.ring.stage_bytes, R.ring.x_bytes};
+    // two CTAs per SM once one per SM cannot run every virtual CTA at the same time (the forms of
+    // k_bicgstab and what they measure: sw2_krylov.cuh)
+    auto pairs = [&](const std::vector<int>& grp) {
+        long long v = 0;
+        for (int k : grp) v += C(k)->krylov_grid;
+        return R.pair_capacity > 0 && v > R.capacity;
+    };
+    auto launch = [&](auto& src, int ctas, bool pair) -> int {
+        using KS = std::decay_t<decltype(src)>;
+        void* kern = pair ? (R.mixed ? krylov_pair_kernel<float, KS>() : krylov_pair_kernel<double, KS>())
+                          : (R.mixed ? krylov_kernel<float, KS>(R.ring.stages) : krylov_kernel<double, KS>(R.ring.stages));
+        void* args[] = {(void*)&src};
+        CK(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kKrylovThreads), args, pair ? R.pair_smem : R.ring.smem, R.stream));
+        R.launches++;
+        return 0;
+    };
     while (j0 < sub.size()) {
         std::vector<int> grp;
-        for (size_t j = j0; j < sub.size() && (int)grp.size() < R.capacity; j++) grp.push_back(sub[j]);
+        const int most = std::max(R.capacity, R.pair_capacity);
+        for (size_t j = j0; j < sub.size() && (int)grp.size() < most; j++) grp.push_back(sub[j]);
         j0 += grp.size();
         if (grp.size() == 1) {
-            const std::vector<int> P = krylov_shares(R, grp);
+            const bool pair = pairs(grp);
+            const std::vector<int> P = krylov_shares(R, grp, pair ? R.pair_capacity : R.capacity);
             KrylovOne one;
             one.Q = R.ktab_h[grp[0]];
             one.rtol = eta[grp[0]];
             one.rtol_dev = R.capturing ? R.eta_dev.p + grp[0] : nullptr;
             one.lay = lay;
-            void* args[] = {(void*)&one};
-            void* kern = R.mixed ? krylov_kernel<float, KrylovOne>(R.ring.stages) : krylov_kernel<double, KrylovOne>(R.ring.stages);
-            CK(cudaLaunchCooperativeKernel(kern, dim3(P[0]), dim3(kKrylovThreads), args, R.ring.smem, R.stream));
-            R.launches++;
+            if ((rc = launch(one, P[0], pair))) return rc;
             continue;
         }
         // rebalancing rounds (host-driven launches only: the host reads which instances paused)
@@ -1010,7 +1043,8 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
         std::vector<int> done(R.ctx.size(), 0);   // iterations a paused solve has behind it
         for (int round = 0; round < rounds; round++) {
             const bool last = round + 1 == rounds;
-            const std::vector<int> P = krylov_shares(R, grp, round ? &done : nullptr);
+            const bool pair = pairs(grp);
+            const std::vector<int> P = krylov_shares(R, grp, pair ? R.pair_capacity : R.capacity, round ? &done : nullptr);
             int total = 0;
             for (int q : P) total += q;
             static thread_local KrylovTab t;   // ~4 KB: not on the stack of every caller
@@ -1033,10 +1067,7 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
                 k_krylov_rearm<<<nblk((int)grp.size(), 128), 128, 0, R.stream>>>(R.ctl.p, t.mp);
                 R.launches++;
             }
-            void* args[] = {(void*)&t};
-            void* kern = R.mixed ? krylov_kernel<float, KrylovTab>(R.ring.stages) : krylov_kernel<double, KrylovTab>(R.ring.stages);
-            CK(cudaLaunchCooperativeKernel(kern, dim3(total), dim3(kKrylovThreads), args, R.ring.smem, R.stream));
-            R.launches++;
+            if ((rc = launch(t, total, pair))) return rc;
             if (last) break;
             CK(cudaMemcpyAsync(R.ctl_h, R.ctl.p, sizeof(KrylovCtl) * R.ctx.size(), cudaMemcpyDeviceToHost, R.stream));
             CK(cudaStreamSynchronize(R.stream));
@@ -2113,7 +2144,7 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
     // every Krylov reduction (an instance's results do not depend on its batch)
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    c->krylov_grid = krylov_vgrid(V, std::min(sms, kMaxVirtual));
+    c->krylov_grid = std::min(krylov_vgrid(V, sms, prm->precision == SW2GPU_MIXED ? kPairRows<float> : kPairRows<double>), kMaxVirtual);
     if (bjacobi) {
         HaloTables ht;
         build_halo(V, c->orowptr_h.data(), ocol.data(), c->krylov_grid, kHaloCapRows, ht);

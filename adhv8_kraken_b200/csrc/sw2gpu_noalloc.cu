@@ -253,7 +253,7 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
     int dev = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bicgstab<double, double, 0, KrylovOne>,
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bicgstab<double, double, kStagesWhole, 1, KrylovOne>,
                                                            kKrylovThreads, 0)) != cudaSuccess)
         return na_fail(SW2GPU_E_CUDA, cudaGetErrorString(e));
     const int grid = krylov_vgrid(nnodes, std::min(sms, kNaVirtual));
@@ -285,7 +285,7 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
     one.rtol_dev = nullptr;
     one.lay = StageLayout{0, 0};
     void* args[] = {(void*)&one};
-    e = cudaLaunchCooperativeKernel((void*)k_bicgstab<double, double, 0, KrylovOne>, dim3(grid),
+    e = cudaLaunchCooperativeKernel((void*)k_bicgstab<double, double, kStagesWhole, 1, KrylovOne>, dim3(grid),
                                                 dim3(kKrylovThreads), args, 0, st);
     if (e != cudaSuccess) return na_fail(SW2GPU_E_CUDA, cudaGetErrorString(e));
     KrylovCtl h;
