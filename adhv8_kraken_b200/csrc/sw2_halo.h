@@ -10,6 +10,9 @@
 // is l, halo row h is (own rows) + h.
 #pragma once
 #include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <utility>
 #include <vector>
 
 namespace sw2 {
@@ -71,6 +74,54 @@ inline void build_halo(int V, const int* rp, const int* col, int vgrid, int cap_
         if (nsub >= most) break;
     }
     t = HaloTables();
+}
+
+// the nodes along the Morton curve of their coordinates: order[new] = old
+inline std::vector<int> morton_order(int V, const double* x, const double* y) {
+    auto spread = [](uint64_t v) {   // a zero between any two of the low 32 bits
+        v = (v | v << 16) & 0x0000ffff0000ffffull;
+        v = (v | v << 8) & 0x00ff00ff00ff00ffull;
+        v = (v | v << 4) & 0x0f0f0f0f0f0f0f0full;
+        v = (v | v << 2) & 0x3333333333333333ull;
+        return (v | v << 1) & 0x5555555555555555ull;
+    };
+    const auto bx = std::minmax_element(x, x + V), by = std::minmax_element(y, y + V);
+    const double x0 = *bx.first, y0 = *by.first, span = std::max(std::max(*bx.second - x0, *by.second - y0), 1e-300);
+    std::vector<std::pair<uint64_t, int>> key(V);
+    for (int i = 0; i < V; i++) {
+        const double fx = (x[i] - x0) / span * 4294967295.0, fy = (y[i] - y0) / span * 4294967295.0;
+        key[i] = {spread((uint64_t)fx) | spread((uint64_t)fy) << 1, i};
+    }
+    std::sort(key.begin(), key.end());
+    std::vector<int> order(V);
+    for (int i = 0; i < V; i++) order[i] = key[i].second;
+    return order;
+}
+
+// The share tables of a mesh.  A numbering without locality has more halo rows than own ones, and every
+// sweep reads each of them from L2 (up to four vectors' entries): the solve then takes the rows in
+// Morton order of their nodes, if that halves the halos.  order[new] = old of that case, else empty;
+// rp, col become the pattern in the order used (blocks of a row stay in the order they had).
+inline void build_shares(int V, std::vector<int>& rp, std::vector<int>& col, const double* x, const double* y, int vgrid,
+                         int cap_rows, HaloTables& t, std::vector<int>& order) {
+    order.clear();
+    build_halo(V, rp.data(), col.data(), vgrid, cap_rows, t);
+    if (t.nsub > 0 && t.idx.size() <= (size_t)V) return;
+    std::vector<int> ord = morton_order(V, x, y), at(V), prp(1, 0), pcol;
+    for (int i = 0; i < V; i++) at[ord[i]] = i;
+    prp.reserve(V + 1);
+    pcol.reserve(col.size());
+    for (int i = 0; i < V; i++) {
+        for (int k = rp[ord[i]]; k < rp[ord[i] + 1]; k++) pcol.push_back(at[col[k]]);
+        prp.push_back((int)pcol.size());
+    }
+    HaloTables p;
+    build_halo(V, prp.data(), pcol.data(), vgrid, cap_rows, p);
+    if (p.nsub == 0 || (t.nsub > 0 && 2 * p.idx.size() > t.idx.size())) return;
+    t = std::move(p);
+    rp.swap(prp);
+    col.swap(pcol);
+    order.swap(ord);
 }
 
 }  // namespace sw2

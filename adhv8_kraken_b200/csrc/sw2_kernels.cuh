@@ -59,6 +59,7 @@ struct __align__(16) Inst {
     double *R, *sol, *jslots, *val, *S, *bs, *dinv;
     void* aoff;                 // folded off-diagonal blocks (MT of the Krylov launch) in tile records
     const int *boff, *orow;     // where tile m's blocks begin (16-byte units), off-diagonal row pointers
+    const int* row;             // the Krylov solve's row of each node (null: its own number)
     unsigned char *ewet, *mark;
     int *glist, *gcount;
     int* ngen;                  // general-list length of the last residual evaluation (the
@@ -854,9 +855,10 @@ __global__ void k_fold_offdiag(const __grid_constant__ Src src) {
         for (int c = 0; c < 3; c++) bq[3 * r + c] = val[(size_t)k * 9 + 3 * r + c] * (S[3 * i + r] * S[3 * j + c]);
 #pragma unroll
     for (int q = 0; q < 9; q++) d[q] = dinv[(size_t)i * 9 + q];
-    const int tile = i / kTileRows;
+    const int r = I.row ? I.row[i] : i, tile = r / kTileRows;
+    const int first = I.row ? I.orow[r] - m.rowptr[i] : -i;   // off-diagonal blocks before row r, less blocks before node i
     MT* o = (MT*)((unsigned char*)I.aoff + 16 * (size_t)I.boff[tile]) +
-            (size_t)(k - i - (k > dp ? 1 : 0) - I.orow[tile * kTileRows]) * 9;
+            (size_t)(k + first - (k > dp ? 1 : 0) - I.orow[tile * kTileRows]) * 9;
     fold_block(d, bq, o);
 }
 

@@ -272,6 +272,9 @@ struct KrylovArgs {
     // staged sweeps (sw2_halo.h): sub-ranges per virtual CTA and their halo rows
     int nsub;
     const int *hptr, *hidx;
+    // node of each row when the solve takes the rows in another order than the nodes (null: row i is
+    // node i); S, bs, Dinv, the state and sol are in node order, everything else in row order
+    const int* order;
     // tile records (TileRecord): where record m and its blocks begin, in 16-byte units from A;
     // null: A holds the blocks in pattern order alone (direct sweeps only)
     const int *toff, *boff;
@@ -745,9 +748,9 @@ __global__ void __launch_bounds__(kKrylovThreads, PER_SM) k_bicgstab(const __gri
             }
             if (mode == kSweepS) return fmadd(-al, ldv(apo + e), ldv(ro + e));
             if (mode == kSweepPlain) return ldv(po + e);
-            const unsigned i = e / 3;   // b = M^-1 b': row e - 3 i of node i's inverse
-            const double* d = KI.Dinv + 3 * (size_t)e;
-            const double* b = K.bs + 3 * i;
+            const unsigned r = e / 3, i = K.order ? __ldg(K.order + r) : r;   // b = M^-1 b': row e - 3 r of node i's inverse
+            const double* d = KI.Dinv + 9 * (size_t)i + 3 * (e - 3 * r);
+            const double* b = K.bs + 3 * (size_t)i;
             return (VT)(d[0] * b[0] + d[1] * b[1] + d[2] * b[2]);
         };
         // first sweep: q . Ap (sum), max |r|; second: As . s, As . As, As . q (sums); at the start:
@@ -1087,10 +1090,11 @@ __global__ void __launch_bounds__(kKrylovThreads, PER_SM) k_bicgstab(const __gri
     // the last iteration set it, else the other copy.
     const VT* ux = KI.vec[C.ucur ^ (conv || pending ? 0 : 1)];
 #pragma unroll 1
-    for (int i = pl * kKrylovRowThreads + tid; i < V; i += np * kKrylovRowThreads) {
-        const double x0 = (double)ldv(ux + 3 * i) * K.S[3 * i];
-        const double x1 = (double)ldv(ux + 3 * i + 1) * K.S[3 * i + 1];
-        const double x2 = (double)ldv(ux + 3 * i + 2) * K.S[3 * i + 2];
+    for (int r = pl * kKrylovRowThreads + tid; r < V; r += np * kKrylovRowThreads) {
+        const int i = K.order ? __ldg(K.order + r) : r;
+        const double x0 = (double)ldv(ux + 3 * r) * K.S[3 * i];
+        const double x1 = (double)ldv(ux + 3 * r + 1) * K.S[3 * i + 1];
+        const double x2 = (double)ldv(ux + 3 * r + 2) * K.S[3 * i + 2];
         if (K.apply_inc) {
             K.u[i] += x0;
             K.v[i] += x1;

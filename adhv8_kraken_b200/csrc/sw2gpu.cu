@@ -186,6 +186,9 @@ struct sw2gpu_ctx {
     // (orowptr / ocol: the BCSR pattern without its diagonal); FP64 or FP32 storage
     std::vector<int> orowptr_h;
     DBuf<int> orowptr, ocol;
+    // the same pattern in the order the Krylov solve takes the rows, where that is not the nodes'
+    // (sw2_halo.h), with the node of each row and the row of each node
+    DBuf<int> krowptr, kcol, korder, krow;
     DBuf<unsigned char> aoff;       // tile records of the folded operator
     DBuf<int> tile_off, blk_off;    // where each begins, and its blocks, in 16-byte units
     DBuf<double> dinv64;
@@ -668,7 +671,8 @@ int runner_tables(Runner& R, int apply_inc) {
         I.S = c->S_.p; I.bs = c->bs.p; I.dinv = c->dinv64.p;
         I.aoff = c->aoff.p;
         I.boff = c->blk_off.p;
-        I.orow = c->orowptr.p;
+        I.orow = c->krowptr.p ? c->krowptr.p : c->orowptr.p;
+        I.row = c->krow.p;
         I.ewet = c->ewet.p; I.mark = c->mark.p; I.glist = c->glist.p; I.gcount = c->gcount.p; I.ngen = c->ngen.p;
         I.npart = c->npart.p; I.norms = R.norms.p + k; I.ncounter = c->ncounter.p; I.singular = R.singular.p + k;
         I.ndir = (int)c->dir_node.size();
@@ -678,8 +682,9 @@ int runner_tables(Runner& R, int apply_inc) {
         KrylovInst& Q = R.ktab_h[k];
         KrylovArgs& A = Q.K;
         A.V = c->V;
-        A.rowptr = c->orowptr.p;
-        A.col = c->ocol.p;
+        A.rowptr = I.orow;
+        A.col = c->kcol.p ? c->kcol.p : c->ocol.p;
+        A.order = c->korder.p;
         A.nsub = c->halo_nsub;
         A.hptr = c->halo_ptr.p;
         A.hidx = c->halo_idx.p;
@@ -2097,23 +2102,6 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
         }
         rc |= up(c->orowptr, orp, st);
         rc |= up(c->ocol, ocol, st);
-        if (bjacobi) {   // the tile records
-            const int nt = nblk(V, kTileRows), esz = prm->precision == SW2GPU_MIXED ? sizeof(float) : sizeof(double);
-            std::vector<int> toff(nt + 1, 0), boff(nt);
-            long long at = 0;
-            for (int m = 0; m < nt; m++) {
-                const int nb = orp[std::min(V, (m + 1) * kTileRows)] - orp[m * kTileRows];
-                const long long bytes = tile_bytes(nb, esz);
-                c->a_cap = (unsigned)std::max<long long>(c->a_cap, std::min<long long>(bytes, 1 << 30));
-                boff[m] = (int)(at + tile_head(nb) / 16);
-                at += bytes / 16;
-                toff[m + 1] = (int)at;
-            }
-            if (at > INT32_MAX) return fail(SW2GPU_E_NOMEM, "the folded operator exceeds 32 GiB");
-            rc |= up(c->tile_off, toff, st);
-            rc |= up(c->blk_off, boff, st);
-            rc |= zalloc(c->aoff, 16 * (size_t)at, st);
-        }
     }
     if (prm->precond == SW2GPU_PREC_BAND) {
         std::vector<int> perm;
@@ -2147,16 +2135,42 @@ int create_impl(const sw2gpu_mesh* m, const sw2gpu_params* prm, void* stream, Me
     c->krylov_grid = std::min(krylov_vgrid(V, sms, prm->precision == SW2GPU_MIXED ? kPairRows<float> : kPairRows<double>), kMaxVirtual);
     if (bjacobi) {
         HaloTables ht;
-        build_halo(V, c->orowptr_h.data(), ocol.data(), c->krylov_grid, kHaloCapRows, ht);
+        std::vector<int> orp = c->orowptr_h, order;
+        build_shares(V, orp, ocol, m->x, m->y, c->krylov_grid, kHaloCapRows, ht, order);
+        if (!order.empty()) {
+            std::vector<int> row(V);
+            for (int i = 0; i < V; i++) row[order[i]] = i;
+            rc |= up(c->krowptr, orp, st);
+            rc |= up(c->kcol, ocol, st);
+            rc |= up(c->korder, order, st);
+            rc |= up(c->krow, row, st);
+            CK(cudaStreamSynchronize(st));   // row goes out of scope
+        }
         c->halo_nsub = ht.nsub;
         c->halo_rows = ht.max_rows;
         rc |= up(c->halo_ptr, ht.ptr, st);
         rc |= up(c->halo_idx, ht.idx, st);
         DBuf<unsigned short> lcol;   // only the records keep it
         rc |= up(lcol, ht.lcol, st);
+        // the tile records
+        const int nt = nblk(V, kTileRows), esz = prm->precision == SW2GPU_MIXED ? sizeof(float) : sizeof(double);
+        std::vector<int> toff(nt + 1, 0), boff(nt);
+        long long at = 0;
+        for (int t = 0; t < nt; t++) {
+            const int nb = orp[std::min(V, (t + 1) * kTileRows)] - orp[t * kTileRows];
+            const long long bytes = tile_bytes(nb, esz);
+            c->a_cap = (unsigned)std::max<long long>(c->a_cap, std::min<long long>(bytes, 1 << 30));
+            boff[t] = (int)(at + tile_head(nb) / 16);
+            at += bytes / 16;
+            toff[t + 1] = (int)at;
+        }
+        if (at > INT32_MAX) return fail(SW2GPU_E_NOMEM, "the folded operator exceeds 32 GiB");
+        rc |= up(c->tile_off, toff, st);
+        rc |= up(c->blk_off, boff, st);
+        rc |= zalloc(c->aoff, 16 * (size_t)at, st);
         if (rc) return rc;
         if (ht.nsub) {
-            k_tile_heads<<<nblk(32LL * nblk(V, kTileRows), 256), 256, 0, st>>>(V, c->orowptr.p, lcol.p, c->tile_off.p, c->aoff.p);
+            k_tile_heads<<<nblk(32LL * nt, 256), 256, 0, st>>>(V, c->krowptr.p ? c->krowptr.p : c->orowptr.p, lcol.p, c->tile_off.p, c->aoff.p);
             CK(cudaGetLastError());
         }
         CK(cudaStreamSynchronize(st));   // the tables go out of scope

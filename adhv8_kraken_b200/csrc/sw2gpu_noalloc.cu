@@ -274,7 +274,7 @@ extern "C" int sw2gpu_bcsr_solve_noalloc(int32_t nnodes, int32_t nnzb, const int
     K.ctl = ctl;
     K.vgrid = grid;
     K.nsub = 0;   // direct sweeps: no share tables
-    K.hptr = K.hidx = nullptr;
+    K.hptr = K.hidx = K.order = nullptr;
     K.toff = K.boff = nullptr;   // blocks in pattern order
     K.spin_limit = 0;   // the library's default bounds on the device waits
     K.copy_limit = 0;
