@@ -212,7 +212,7 @@ struct sw2gpu_ctx {
     DBuf<int> halo_ptr, halo_idx;
     // autotuned launch variants (sw2gpu_autotune): they change speed, never results
     int tune_jac_minb = 2;          // wet-Jacobian CTAs per SM the register budget is cut for
-    int tune_stages = -1;           // Krylov tile-ring depth (0: sweeps from global memory; -1: by occupancy)
+    int tune_stages = -1;           // Krylov tile-ring depth (0: sweeps from global memory; -1: the deepest that fits)
     // polls of a Krylov grid-barrier / tile-copy wait before it gives up (0: the library's
     // defaults); sw2gpu_set_wait_limits
     long long wait_barrier = 0, wait_copy = 0;
@@ -836,7 +836,7 @@ int launch_jacobian(Runner& R, const std::vector<int>& sub, bool differences = f
                 <<<std::min(nb_, R.jac_ctas[MB - 1]), th_, kJacWetSmem, R.stream>>>(src, nb_);
         });
     };
-    if (!R.jac_ctas[R.jac_minb - 1])
+    if (!diff.empty() && !R.jac_ctas[R.jac_minb - 1])
         return fail(SW2GPU_E_CUDA, "wet-Jacobian variant %d does not fit on this device", R.jac_minb);
     rc = R.jac_minb == 1 ? wet(std::integral_constant<int, 1>{}) : wet(std::integral_constant<int, 2>{});
     if (rc) return rc;
@@ -3003,7 +3003,8 @@ int sw2gpu_get_variant(const sw2gpu_ctx* c, int32_t* jac_minb, int32_t* stages) 
 }
 
 // Times every launch variant on the context's own mesh and current state and keeps the
-// fastest: the wet-Jacobian register budget (1 or 2 CTAs per SM) and the Krylov tile-ring
+// fastest: the register budget of the differenced wet Jacobian (1 or 2 CTAs per SM; left alone where
+// the steps use the closed forms and never launch it) and the Krylov tile-ring
 // depth (0, 2 or 3 stages).  The variants compute the same bits; the state is left as found.
 int sw2gpu_autotune(sw2gpu_ctx* c, int32_t* jac_minb, int32_t* stages) {
     if (!c) return fail(SW2GPU_E_ARG, "null context");
@@ -3041,7 +3042,7 @@ int sw2gpu_autotune(sw2gpu_ctx* c, int32_t* jac_minb, int32_t* stages) {
     int best_j = c->tune_jac_minb;
     float tb = 1e30f;
     for (int m : {1, 2}) {
-        if (!R.jac_ctas[m - 1]) continue;   // does not fit on this device
+        if (c->wet_closed || !R.jac_ctas[m - 1]) continue;   // not used, or does not fit on this device
         R.jac_minb = m;
         float t = 1e30f;
         if ((rc = timed([&] { return launch_jacobian(R, one); }, t))) break;

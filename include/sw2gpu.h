@@ -158,9 +158,11 @@ int sw2gpu_remesh(sw2gpu_ctx *old, const sw2gpu_mesh *mesh, sw2gpu_ctx **out);
  * or 2 resident CTAs per SM; Newton iterations differentiate fully wet elements of materials
  * with isotropic user viscosity in closed form and do not launch it) and the depth of the
  * Krylov kernel's shared-memory tile rings (stages: 0 = sweeps read global memory, 2 or 3 = one
- * or two places per group of row warps).  sw2gpu_autotune times every variant on the
- * context's own mesh and current state (which it leaves as it found it) and keeps the
- * fastest; a batch uses the variants of its instance with the most blocks. */
+ * or two places per group of row warps; launches that put two CTAs on an SM, which batches and
+ * large meshes are, have rings of a depth of their own unless it is 0).  sw2gpu_autotune times the
+ * variants on the context's own mesh and current state (which it leaves as it found it) and keeps the
+ * fastest; jac_minb stays as it was where no step would launch that kernel.  A batch uses the variants
+ * of its instance with the most blocks. */
 int sw2gpu_autotune(sw2gpu_ctx *ctx, int32_t *jac_minb, int32_t *stages);
 int sw2gpu_set_variant(sw2gpu_ctx *ctx, int32_t jac_minb, int32_t stages);
 int sw2gpu_get_variant(const sw2gpu_ctx *ctx, int32_t *jac_minb, int32_t *stages);
