@@ -118,6 +118,8 @@ struct SrcPar {
 // at all three levels is positive with a margin no finite-difference perturbation of h
 // (|eps| <= max(1.5e-8, 1.5e-8 |h|)) can cross; every other element goes on the list.
 constexpr double kWetMargin = 1e-6;
+// the closed-form Jacobian (sw2_wet_jac.cuh) leaves out the floors under the mean depth
+static_assert(kWetMargin > kNotQuiteSmall && kWetMargin > kDragDepthFloor, "wet elements lie above the depth floors");
 
 __device__ __forceinline__ void load_elem(const DevMesh& m, const State& s, int e, int rule_vel, ElemIn& in, int* n,
                                           int* df) {

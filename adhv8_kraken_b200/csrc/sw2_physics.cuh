@@ -230,8 +230,9 @@ __device__ __forceinline__ double wd_average(const ClipGeo& c, const double* x, 
     return f;
 }
 
+constexpr double kDragDepthFloor = 1.E-8;
 __device__ __forceinline__ double drag_coef(double depth, double ks) {  // fr_bedshstr_drag_coef.c:18-40
-    depth = fmax(depth, 1.E-8);
+    depth = fmax(depth, kDragDepthFloor);
     ks = fmax(ks, 1.E-8);
     double rh = (ks > 29.7 * depth) ? 1. / 29.7 : depth / ks;
     double bta = 29.7 * rh;

@@ -7,6 +7,9 @@
 // gradients, drag law and SUPG scales once per element, a dozen products per entry after that.
 // The kinks -- the depth floors max(h, dll) and max(h, dul) -- are differenced with the reference's
 // step, so a depth that sits exactly on one gives the reference's mean of the two sides.
+// The floors under the mean depth in the residual's quotients (FLT_EPSILON and the drag law's 1e-8) are
+// left out: an element is on this path only while every depth is above kWetMargin (sw2_kernels.cuh),
+// which is higher; thinner films take the general path and its differences.
 //
 // Used by the Newton iterations of instances whose materials have an isotropic user eddy viscosity
 // (the estimated viscosities have a root of the velocity gradients, which is not smooth at rest);
