@@ -562,13 +562,13 @@ __global__ void __launch_bounds__(kJacWetThreads, MINB) k_jac_elem_wet(const __g
 }
 
 // Fully wet elements by the closed forms of sw2_wet_jac.cuh, one thread per element, for instances
-// whose materials they cover.  Bound: writing the element blocks (648 B per triangle; 0.10 ms of the
-// 1M-triangle basin at the measured copy rate) and FP64 latency (about 1,500 products per element in
-// one thread).  The 81 entries go through shared memory (odd stride: no bank conflicts), so the
+// whose materials they cover.  Bound: FP64 latency -- about 1,500 products per element in one thread of
+// 255 registers, so 12 % of the warps are active: 0.193 ms for 600k triangles, at 26 % of the DRAM
+// throughput (writing the element blocks alone, 648 B per triangle, would take 0.06 ms at the measured
+// copy rate).  The 81 entries go through shared memory (odd stride: no bank conflicts), so the
 // records leave as one contiguous stream; records of elements off the wet path are left for the
 // general launch that follows.  Jacobian phase of the 1M-triangle basin (this, the general elements and
-// the gather): 0.68 ms per Newton iteration, 2.28 with the eighteen
-// differenced residuals.
+// the gather): 0.59 ms per Newton iteration, 2.28 with the eighteen differenced residuals.
 constexpr int kJacClosedElems = 64;
 template <class Src>
 __global__ void __launch_bounds__(kJacClosedElems) k_jac_elem_closed(const __grid_constant__ Src src) {

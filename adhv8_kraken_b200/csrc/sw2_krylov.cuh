@@ -21,6 +21,7 @@
 //     (and, in the first sweep, updated) once instead of once per neighbour;
 //   - an iteration's vector update is part of the next iteration's first sweep, so an iteration
 //     is two sweeps and two grid barriers;
+//   - the rows are taken in an order with locality, the nodes' own where it has it (sw2_halo.h);
 //   - the matrix does not change during a solve, so the copy warp streams its tiles without
 //     regard to the barriers, and a CTA whose tiles all fit in its ring fetches them once per solve.
 // A batch launch may stop the instances still iterating at an iteration boundary once enough
@@ -398,9 +399,8 @@ static __global__ void k_krylov_rearm(KrylovCtl* ctl, const __grid_constant__ La
 }
 
 // ---- tile staging: one bulk copy per tile, completion on an mbarrier -------------------------
-// Tile m = node rows [m kTileRows, (m+1) kTileRows); its blocks and column indices are contiguous.
-// The copied ranges are rounded out to 16 bytes (the bulk-copy rule); the arrays are allocated
-// with 16 spare bytes and start on 256-byte boundaries, so the rounded ranges stay inside them.
+// Tile m = rows [m kTileRows, (m+1) kTileRows) of the solve; its record begins and ends on 16-byte
+// boundaries (the bulk-copy rule).
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {

@@ -1010,12 +1010,15 @@ int launch_linear(Runner& R, const std::vector<int>& all, const std::vector<doub
     // instances that cannot all be co-resident go in successive launches
     size_t j0 = 0;
     const StageLayout lay{R.ring.stage_bytes, R.ring.x_bytes};
-    // two CTAs per SM once one per SM cannot run every virtual CTA at the same time (the forms of
-    // k_bicgstab and what they measure: sw2_krylov.cuh)
+    // two CTAs per SM where there are more than 5/4 virtual CTAs per SM (the forms of k_bicgstab and
+    // what they measure: sw2_krylov.cuh).  Below, one per SM: a CTA that runs two keeps the tiles of
+    // both in its ring (Krylov ms of an engine, one and two per SM: 4 members of 38 virtual CTAs each
+    // 7.3 and 8.4, of 45 7.5 and 8.5, of 50 5.3 and 5.1; 2 members of 75 4.9 and 4.3, of 100 4.9 and
+    // 4.0; 3 of 100 7.4 and 5.8).  More members than SMs have no other way.
     auto pairs = [&](const std::vector<int>& grp) {
         long long v = 0;
         for (int k : grp) v += C(k)->krylov_grid;
-        return R.pair_capacity > 0 && v > R.capacity;
+        return R.pair_capacity > 0 && (4 * v > 5 * R.capacity || (int)grp.size() > R.capacity);
     };
     auto launch = [&](auto& src, int ctas, bool pair) -> int {
         using KS = std::decay_t<decltype(src)>;

@@ -637,18 +637,18 @@ def run_ours(args, rank, world, local_rank, ens_models=None, serve=None):
     lin = sum(s["linear_its"] for s in stats)
     nnzb = g.nnzb
     hbm, src = peaks()
-    # algorithmic bytes per launch.  FD Jacobian: element inputs + node state + 81 outputs per
+    # algorithmic bytes per launch.  Jacobian: element inputs + node state + 81 outputs per
     # triangle.  BiCGSTAB on the folded operator (block-Jacobi inverse multiplied into the
-    # off-diagonal blocks, identity diagonal): per iteration two sweeps over the nnzb - V
-    # off-diagonal blocks (72 B values + 4 B column) and the row pointers, plus 16 vector
-    # streams of 3 doubles per node (sweep 1: q, p in, Ap out; sweep 2: r, Ap, q in, As out;
-    # update: r, Ap, u, p, As in, u, r, p, best-u out).  Per launch once: b' and the inverses
-    # in, b and u out (prologue), one more sweep with b, u in and r, q, p, Ap out, and the
-    # exit pass (u and S in, state in and out, solution out).
+    # off-diagonal blocks, identity diagonal): per iteration two sweeps over the tile records (72 B
+    # values + 2 B column per off-diagonal block, row pointers and padding per 32 rows) and 14 vector
+    # streams of 3 doubles per node (sweep 1: Ap, p, r, As, u, q in, u, r, p, Ap out; sweep 2: r, Ap, q
+    # in, As out; the halo rows read again, a few per cent, are not counted).  Per launch once: b' and
+    # the inverses in, u out, one sweep with r, q, p out, one with p, q in and Ap out, and the exit
+    # pass (u and S in, state in and out, solution out).
     jac_bytes = T * (3 * 4 + 7 * 8 + 4 + 4 + 1) + V * 12 * 8 + T * 81 * 8
-    sweep_bytes = (nnzb - V) * (9 * 8 + 4) + (V + 1) * 4
-    kry_iter_bytes = 2 * sweep_bytes + V * 24 * 16
-    kry_launch_bytes = V * (24 + 72 + 48) + sweep_bytes + V * 24 * 6 + V * (48 + 48 + 24)
+    sweep_bytes = (nnzb - V) * (9 * 8 + 2) + (V + 31) // 32 * 96
+    kry_iter_bytes = 2 * sweep_bytes + V * 24 * 14
+    kry_launch_bytes = V * (24 + 72 + 24) + 2 * sweep_bytes + V * 24 * 6 + V * (48 + 48 + 24)
     kernels = {
         "k_jac_elem": (jac, newton, jac_bytes),
         "k_bicgstab": (kry, newton, kry_iter_bytes * (lin / max(newton, 1)) + kry_launch_bytes),
