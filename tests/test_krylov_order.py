@@ -104,8 +104,9 @@ def test_a_scattered_numbering_is_reordered(lib, nx, ny, vgrid):
             assert np.array_equal(rows[lcol[krp[r0]:krp[r1]]], kcol[krp[r0]:krp[r1]])
 
 
-@pytest.mark.parametrize("nx,ny,vgrid", [(300, 12, 22), (64, 64, 4), (9, 9, 1)])
+@pytest.mark.parametrize("nx,ny,vgrid", [(300, 12, 22), (64, 64, 4), (9, 9, 1), (55, 47, 41)])
 def test_a_numbering_with_locality_is_kept(lib, nx, ny, vgrid):
+    """The last one has more halo than own rows, but few of either."""
     rp, col, x, y = _grid(nx, ny, np.arange(nx * ny))
     nsub, _, krp, kcol, order, _, idx, _, before = _call(lib, rp, col, x, y, vgrid, 1024)
     assert nsub >= 1 and len(order) == 0 and len(idx) == before
