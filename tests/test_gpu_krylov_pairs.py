@@ -82,3 +82,31 @@ def test_one_launch_per_solve_above_one_member_per_sm():
         for g in gs:
             g.close()
     assert launches[0] == launches[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [capi.SW2GPU_FP64, capi.SW2GPU_MIXED])
+@pytest.mark.parametrize("rebalance", [(4, 0.5), (8, 0.0)], ids=["default", "every-iteration"])
+def test_paused_solves_go_on_in_either_form(precision, rebalance):
+    """An engine whose solves pause: a launch of two CTAs per SM resumes in another, and the last few
+    members in launches of one per SM; each ends where it ends alone."""
+    models = [_basin(n, 60 + k) for k, n in enumerate((900, 5000, 7001, 9000, 13000, 15001))]
+    alone = []
+    for m in models:
+        g = SW2GPU(m, precision=precision)
+        g.step()
+        alone.append(_state(g))
+        g.close()
+    solvers = [SW2GPU(m, precision=precision) for m in models]
+    eng = SW2Engine(precision)
+    eng.set_rebalance(*rebalance)
+    for g in solvers:
+        eng.add(g, 1)
+    done = eng.run()
+    assert len(done) == len(models) and all(d["status"] == 0 for d in done)
+    for g, want in zip(solvers, alone):
+        for a, b in zip(_state(g), want):
+            assert np.array_equal(a, b)
+    eng.close()
+    for g in solvers:
+        g.close()
